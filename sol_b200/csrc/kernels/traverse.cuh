@@ -78,19 +78,36 @@ __device__ __forceinline__ Vec3 tri_vertex(float4 a) { return vec3(a.x, a.y, a.z
 __device__ __forceinline__ float fminf3(float a, float b, float c) { return fminf(fminf(a, b), c); }
 __device__ __forceinline__ float fmaxf3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
 
+/// (lo - o) * id and (hi - o) * id, both planes of a slab in one packed subtract
+/// and one packed multiply (sm_100's two-wide FP32 forms, each half rounded as
+/// the scalar operation, so the same bits in half the issue slots).  A packed
+/// multiply must not feed a packed add here: ptxas contracts that pair into a
+/// fused multiply-add whatever -fmad says.
+__device__ __forceinline__ void slab_planes(float lo, float hi, float o, float id, float& t_lo, float& t_hi) {
+    asm("{\n\t.reg .b64 p, q, r;\n\t"
+        "mov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %4};\n\tmov.b64 r, {%5, %5};\n\t"
+        "sub.rn.f32x2 p, p, q;\n\tmul.rn.f32x2 p, p, r;\n\tmov.b64 {%0, %1}, p;\n\t}"
+        : "=f"(t_lo), "=f"(t_hi) : "f"(lo), "f"(hi), "f"(o), "f"(id));
+}
+
 /// Entry and (widened) exit distances of a ray against both child boxes of a
 /// node: a = c0.x and c0.y bounds, b = c1.x and c1.y bounds, c = both z bounds.
 /// (bound - org) * (1/dir) takes two correctly rounded operations per plane, so
 /// the widened exit distance stays conservative even for grazing rays (the
-/// product-with-offset form loses |org / dir| ulps to cancellation).
+/// product-with-offset form loses |org / dir| ulps to cancellation).  The
+/// traversal kernels are bound by instruction issue at about 9 of 32 lanes per
+/// node step, and the 24 scalar subtracts and multiplies were the largest
+/// share of a step; packed they are 12 (1M-triangle frame, 64 samples: 50.4 ->
+/// 46.6 ms together with the fused index check of Traversal::run).
 __device__ __forceinline__ void child_slabs(float4 a, float4 b, float4 c, Vec3 org, Vec3 idir, float tmin,
                                             float tmax, float& n0, float& f0, float& n1, float& f1) {
-    const float t0lx = (a.x - org.x) * idir.x, t0hx = (a.y - org.x) * idir.x;
-    const float t0ly = (a.z - org.y) * idir.y, t0hy = (a.w - org.y) * idir.y;
-    const float t0lz = (c.x - org.z) * idir.z, t0hz = (c.y - org.z) * idir.z;
-    const float t1lx = (b.x - org.x) * idir.x, t1hx = (b.y - org.x) * idir.x;
-    const float t1ly = (b.z - org.y) * idir.y, t1hy = (b.w - org.y) * idir.y;
-    const float t1lz = (c.z - org.z) * idir.z, t1hz = (c.w - org.z) * idir.z;
+    float t0lx, t0hx, t0ly, t0hy, t0lz, t0hz, t1lx, t1hx, t1ly, t1hy, t1lz, t1hz;
+    slab_planes(a.x, a.y, org.x, idir.x, t0lx, t0hx);
+    slab_planes(a.z, a.w, org.y, idir.y, t0ly, t0hy);
+    slab_planes(c.x, c.y, org.z, idir.z, t0lz, t0hz);
+    slab_planes(b.x, b.y, org.x, idir.x, t1lx, t1hx);
+    slab_planes(b.z, b.w, org.y, idir.y, t1ly, t1hy);
+    slab_planes(c.z, c.w, org.z, idir.z, t1lz, t1hz);
     n0 = fmaxf3(fminf(t0lx, t0hx), fminf(t0ly, t0hy), fmaxf(fminf(t0lz, t0hz), tmin));
     f0 = fminf3(fmaxf(t0lx, t0hx), fmaxf(t0ly, t0hy), fminf(fmaxf(t0lz, t0hz), tmax)) * kSlabWiden;
     n1 = fmaxf3(fminf(t1lx, t1hx), fminf(t1ly, t1hy), fmaxf(fminf(t1lz, t1hz), tmin));
@@ -151,10 +168,11 @@ struct Traversal {
                                         TraversalCounters& ctr, uint32_t num_nodes, uint32_t num_tris,
                                         uint32_t max_steps, unsigned int* fault, Stack& stack, int min_active) {
         while (node != kStackSentinel) {
-            // Descend inner nodes until a leaf (or the end) is reached.
-            while (node >= 0) {
+            // Descend inner nodes until a leaf, the end or a reference outside the
+            // node array is reached: as unsigned numbers leaf references and the
+            // sentinel lie above every node index, so one comparison decides.
+            while ((uint32_t)node < num_nodes) {
                 if (++steps > max_steps) return fail(fault, kFaultTraversalSteps);
-                if ((uint32_t)node >= num_nodes) return fail(fault, kFaultNodeIndex);
                 const DNode* n = nodes + node;
                 const float4 a = ldg4(n->b0);
                 const float4 b = ldg4(n->b1);
@@ -180,6 +198,7 @@ struct Traversal {
                 }
             }
             if (node == kStackSentinel) break;
+            if (node >= 0) return fail(fault, kFaultNodeIndex);
             // Leaf: ~node = (first << 3) | (count - 1)
             const uint32_t v = ~(uint32_t)node;
             const uint32_t first = v >> 3, count = (v & 7u) + 1u;
