@@ -83,7 +83,7 @@ cudaError_t upload(T** dst, const std::vector<T>& src) {
 void release(SolGpuScene* s) {
     if (!s) return;
     DeviceGuard g(s->device);
-    cudaFree(s->nodes); cudaFree(s->tris); cudaFree(s->shade); cudaFree(s->bsdfs);
+    cudaFree(s->boxes); cudaFree(s->tris); cudaFree(s->shade); cudaFree(s->bsdfs);
     cudaFree(s->textures); cudaFree(s->images); cudaFree(s->texels); cudaFree(s->lights);
     cudaFree(s->counters); cudaFree(s->film_tmp); cudaFree(s->split_scratch); cudaFree(s->adj_texels4); cudaFree(s->param_offsets); cudaFree(s->fault);
     if (s->film_host) cudaFreeHost(s->film_host);
@@ -226,6 +226,7 @@ int sol_gpu_scene_create_ex(const SolGpuSceneDesc* desc, int device, uint32_t fl
         up(reinterpret_cast<void**>(&d_i), desc->indices, sizeof(uint32_t) * 3 * nt);
         up(reinterpret_cast<void**>(&d_b), desc->tri_bsdf, sizeof(int32_t) * nt);
         up(reinterpret_cast<void**>(&d_l), desc->tri_light, sizeof(int32_t) * nt);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);   // the build's stream does not wait for the copies
         LbvhResult r;
         if (e == cudaSuccess) e = build_lbvh(d_v, d_i, d_n, d_uv, d_b, d_l, nt, s->stream, &r);
         cudaEventRecord(b1, s->stream);
@@ -235,6 +236,7 @@ int sol_gpu_scene_create_ex(const SolGpuSceneDesc* desc, int device, uint32_t fl
         cudaEventDestroy(b1);
         cudaFree(d_v); cudaFree(d_n); cudaFree(d_uv); cudaFree(d_i); cudaFree(d_b); cudaFree(d_l);
         if (e == cudaSuccess) {
+            s->boxes = r.boxes;
             s->nodes = r.nodes;
             s->tris = r.tris;
             s->shade = r.shade;
@@ -250,7 +252,15 @@ int sol_gpu_scene_create_ex(const SolGpuSceneDesc* desc, int device, uint32_t fl
         }
     }
     if (!gpu_bvh) {
-        if (e == cudaSuccess) e = upload(&s->nodes, flat.nodes);
+        const size_t n = flat.nodes.size();
+        if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&s->boxes), n * (sizeof(DBoxNode) + sizeof(DNode)));
+        if (e == cudaSuccess) {
+            s->nodes = reinterpret_cast<DNode*>(s->boxes + n);
+            e = cudaMemcpy(s->nodes, flat.nodes.data(), n * sizeof(DNode), cudaMemcpyHostToDevice);
+        }
+        // On the stream of the copy: a copy from pageable memory may return before its
+        // data has reached the device, and other streams do not wait for it.
+        if (e == cudaSuccess) e = launch_pack_boxes(s->nodes, (uint32_t)n, s->boxes, cudaStreamLegacy);
         if (e == cudaSuccess) e = upload(&s->tris, flat.tris);
         if (e == cudaSuccess) e = upload(&s->shade, flat.shade);
     }
@@ -283,9 +293,11 @@ int sol_gpu_scene_create_ex(const SolGpuSceneDesc* desc, int device, uint32_t fl
         std::vector<unsigned long long> offs(s->texture_offsets.begin(), s->texture_offsets.end());
         if (e == cudaSuccess) e = upload(&s->param_offsets, offs);
     }
+    // The uploads (and the box nodes made from them) are on the legacy stream, renders on any.
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (e != cudaSuccess) { int rc = cuda_fail(e, "scene upload"); release(s); return rc; }
 
-    s->view.nodes = s->nodes;
+    s->view.boxes = s->boxes;
     s->view.tris = s->tris;
     s->view.shade = s->shade;
     s->view.bsdfs = s->bsdfs;
@@ -310,7 +322,7 @@ int sol_gpu_scene_create_ex(const SolGpuSceneDesc* desc, int device, uint32_t fl
     s->info.num_nodes = (uint32_t)flat.nodes.size();
     s->info.bvh_depth = flat.depth;
     s->info.sah_cost = flat.sah_cost;
-    s->info.device_bytes = flat.nodes.size() * sizeof(DNode) + num_tris * (sizeof(DTri) + sizeof(DTriShade));
+    s->info.device_bytes = flat.nodes.size() * (sizeof(DBoxNode) + sizeof(DNode)) + num_tris * (sizeof(DTri) + sizeof(DTriShade));
     s->info.build_ms = (float)flat.build_ms + gpu_build_ms;
 #if SOL_L2_PERSIST
     // Keep the upper BVH levels (stored first) in L2: raise this process's
@@ -327,7 +339,7 @@ int sol_gpu_scene_create_ex(const SolGpuSceneDesc* desc, int device, uint32_t fl
             cudaDeviceGetLimit(&have, cudaLimitPersistingL2CacheSize);
             const size_t bytes = (size_t)flat.top_nodes * sizeof(DNode);
             if (have > 0 && bytes > 0) {
-                s->l2.base = s->nodes;
+                s->l2.base = s->boxes;
                 s->l2.bytes = bytes;
                 s->l2.hit_ratio = (float)std::min(1.0, (double)have / (double)bytes);
             }

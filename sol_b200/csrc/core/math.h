@@ -445,11 +445,11 @@ SOL_HD void edge_functions(const RayShear& r, Vec3 a, Vec3 b, Vec3 c,
 }
 
 /// Watertight intersection of a ray with triangle (v0, v1, v2), both sides.
-/// On a hit strictly inside (tmin, tmax) returns true with the distance `t`
+/// On a hit with tmin < t <= tmax returns true with the distance `t`
 /// (in units of the ray direction) and barycentrics u (weight of v1) and v
 /// (weight of v2).
-SOL_HD bool intersect_triangle(const RayShear& r, Vec3 v0, Vec3 v1, Vec3 v2,
-                               float tmin, float tmax, float* t_out, float* u_out, float* v_out) {
+SOL_HD bool intersect_triangle_upto(const RayShear& r, Vec3 v0, Vec3 v1, Vec3 v2,
+                                    float tmin, float tmax, float* t_out, float* u_out, float* v_out) {
     Vec3 a = v0 - r.org, b = v1 - r.org, c = v2 - r.org;
     float U, V, W, az, bz, cz;
     edge_functions(r, a, b, c, &U, &V, &W, &az, &bz, &cz);
@@ -459,10 +459,21 @@ SOL_HD bool intersect_triangle(const RayShear& r, Vec3 v0, Vec3 v1, Vec3 v2,
     float T = U * az + V * bz + W * cz;
     float rcp = 1.0f / det;
     float t = T * rcp;
-    if (!(t > tmin && t < tmax)) return false;
+    if (!(t > tmin && t <= tmax)) return false;
     *t_out = t;
     *u_out = V * rcp;
     *v_out = W * rcp;
+    return true;
+}
+
+/// intersect_triangle_upto for hits strictly inside (tmin, tmax).
+SOL_HD bool intersect_triangle(const RayShear& r, Vec3 v0, Vec3 v1, Vec3 v2,
+                               float tmin, float tmax, float* t_out, float* u_out, float* v_out) {
+    float t, u, v;
+    if (!intersect_triangle_upto(r, v0, v1, v2, tmin, tmax, &t, &u, &v) || !(t < tmax)) return false;
+    *t_out = t;
+    *u_out = u;
+    *v_out = v;
     return true;
 }
 

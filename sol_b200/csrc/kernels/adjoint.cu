@@ -405,10 +405,10 @@ __device__ SOL_ADJ_OUTLINE int trace_recorded(const SceneView& s, const DConfig&
         VertexOut vo;
         shade_vertex(s, cfg, light_pick_prob, slot, t, ps, vo, recd, true, hu, hv);
         if (vo.has_shadow) {
-            float smax = 1.0f - cfg.ray_offset;
-            const int occ = traverse<true, false>(s, vo.sh_org, vo.sh_dir, cfg.ray_offset, smax, tc);
+            const bool occ =
+                occluded<false>(s, vo.sh_org, vo.sh_dir, cfg.ray_offset, 1.0f - cfg.ray_offset, tc, stack);
             ++n_rays;
-            if (occ < 0) {
+            if (!occ) {
                 ps.color = ps.color + vo.pending;
                 recd.R->flags |= kNee;
             }

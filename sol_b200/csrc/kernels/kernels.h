@@ -46,7 +46,7 @@ constexpr int kMegakernelViewsMinBlocks = SOL_MEGAKERNEL_VIEWS_MIN_BLOCKS;
 /// K1 renders with at least this many paths per resident lane of the
 /// full-occupancy build use it; smaller renders use the 12-block build.
 constexpr uint64_t kMegakernelFullPathsPerLane = 8;
-constexpr int kTraceBlock = 128;
+constexpr int kTraceBlock = 64;
 #ifndef SOL_SPLIT_SCRATCH_MAX_MB
 #define SOL_SPLIT_SCRATCH_MAX_MB 2048
 #endif

@@ -138,11 +138,11 @@ pt_megakernel(SceneView s, DCamera cam, DConfig cfg, uint64_t sample_index, uint
 
         // --- shadow ray of this vertex (path_tracer.cpp:72-74) -------------
         if (vo.has_shadow) {
-            float smax = 1.0f - cfg.ray_offset;
-            const int occ = traverse<true, kCount>(s, vo.sh_org, vo.sh_dir, cfg.ray_offset, smax, tc, stack);
+            const bool occ =
+                occluded<kCount>(s, vo.sh_org, vo.sh_dir, cfg.ray_offset, 1.0f - cfg.ray_offset, tc, stack);
             ++n_rays;
             ++n_shadow;
-            if (occ < 0) ps.color = ps.color + vo.pending;
+            if (!occ) ps.color = ps.color + vo.pending;
         }
 
         bool end = vo.end;
@@ -242,12 +242,11 @@ pt_megakernel_lean(SceneView s, DCamera cam, DConfig cfg, uint64_t sample_index,
                     shade_vertex<kBasic>(s, cfg, light_pick_prob, slot, t, ps, vo, true, hu, hv);
                     // shadow ray of this vertex (path_tracer.cpp:72-74)
                     if (vo.has_shadow) {
-                        float smax = 1.0f - cfg.ray_offset;
-                        const int occ =
-                            traverse<true, false>(s, vo.sh_org, vo.sh_dir, cfg.ray_offset, smax, tc, stack);
+                        const bool occ =
+                            occluded<false>(s, vo.sh_org, vo.sh_dir, cfg.ray_offset, 1.0f - cfg.ray_offset, tc, stack);
                         ++n_rays;
                         ++n_shadow;
-                        if (occ < 0) ps.color = ps.color + vo.pending;
+                        if (!occ) ps.color = ps.color + vo.pending;
                     }
                     if (vo.end) end = true;
                     else end = ++ps.path_len >= cfg.max_path_len;
@@ -287,11 +286,11 @@ pt_megakernel_lean(SceneView s, DCamera cam, DConfig cfg, uint64_t sample_index,
             shade_vertex<kBasic>(s, cfg, light_pick_prob, slot, t, ps, vo, true, hu, hv);
             // shadow ray of this vertex (path_tracer.cpp:72-74)
             if (vo.has_shadow) {
-                float smax = 1.0f - cfg.ray_offset;
-                const int occ = traverse<true, false>(s, vo.sh_org, vo.sh_dir, cfg.ray_offset, smax, tc, stack);
+                const bool occ =
+                    occluded<false>(s, vo.sh_org, vo.sh_dir, cfg.ray_offset, 1.0f - cfg.ray_offset, tc, stack);
                 ++n_rays;
                 ++n_shadow;
-                if (occ < 0) ps.color = ps.color + vo.pending;
+                if (!occ) ps.color = ps.color + vo.pending;
             }
             if (vo.end) break;
             ++ps.path_len;
@@ -419,11 +418,11 @@ pt_megakernel_views(const WfView* __restrict__ views, uint32_t num_views, uint32
         vo.end = slot < 0;
         if (!vo.end) shade_vertex<kBasic>(*s, cfg, light_pick_prob, slot, t, ps, vo, true, hu, hv);
         if (vo.has_shadow) {
-            float smax = 1.0f - cfg.ray_offset;
-            const int occ = traverse<true, kCount>(*s, vo.sh_org, vo.sh_dir, cfg.ray_offset, smax, tc, stack);
+            const bool occ =
+                occluded<kCount>(*s, vo.sh_org, vo.sh_dir, cfg.ray_offset, 1.0f - cfg.ray_offset, tc, stack);
             ++n_rays;
             ++n_shadow;
-            if (occ < 0) ps.color = ps.color + vo.pending;
+            if (!occ) ps.color = ps.color + vo.pending;
         }
         bool end = vo.end;
         if (!end) {

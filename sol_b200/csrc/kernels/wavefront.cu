@@ -253,7 +253,7 @@ template <bool kAnyHit, class Fetch, class Finish>
 __device__ __forceinline__ void trace_queue(const WfSceneTable& scenes, uint32_t n, uint32_t* fetch_counter,
                                             int refill_below, Fetch fetch, Finish finish,
                                             unsigned long long& rays) {
-    Traversal<kAnyHit, false, true> tr;
+    Traversal<kAnyHit, false, true, false> tr;
     WfStack stack = make_stack();
     const SceneView* sv = &scenes.v[0];
     uint32_t at = 0;
@@ -283,8 +283,9 @@ __device__ __forceinline__ void trace_queue(const WfSceneTable& scenes, uint32_t
         }
         if (!__any_sync(0xffffffffu, has)) break;
         // Once the queue is drained there is nothing to refill: run to the end.
-        if (has && tr.run(sv->nodes, sv->tris, tc, sv->num_nodes, sv->num_tris, sv->max_steps, sv->fault, stack,
-                          more ? refill_below : 0)) {
+        if (has && tr.run(nullptr, sv->boxes, sv->tris, tc, sv->num_nodes, sv->num_tris, sv->max_steps, sv->fault,
+                          stack, more ? refill_below : 0)) {
+            tr.resolve(*sv, kFloatMax);
             finish(at, tr);
             has = false;
         }
@@ -303,13 +304,13 @@ wf_extend(const WfParams* __restrict__ Pp, const __grid_constant__ WfSceneTable 
     const float4* __restrict__ ro = P.ray_o[p];
     const float4* __restrict__ rd = P.ray_d[p];
     unsigned long long rays = 0;
-    auto fetch = [&](uint32_t i, Traversal<false, false, true>& tr, WfStack& stack) -> uint32_t {
+    auto fetch = [&](uint32_t i, Traversal<false, false, true, false>& tr, WfStack& stack) -> uint32_t {
         const float4 o = ro[i], d = rd[i];
         const uint32_t scene = __float_as_uint(d.w) >> kWfSlotBits;
         tr.start(vec3(o.x, o.y, o.z), vec3(d.x, d.y, d.z), o.w, kFloatMax, scenes.v[scene].num_tris > 0, stack);
         return scene;
     };
-    auto finish = [&](uint32_t i, const Traversal<false, false, true>& tr) {
+    auto finish = [&](uint32_t i, const Traversal<false, false, true, false>& tr) {
         P.hit[i] = make_float4(__int_as_float(tr.hit), tr.tmax, tr.hu, tr.hv);
         if (sort) {
             int kind = kWfBins - 1;
@@ -424,13 +425,13 @@ wf_shadow(const WfParams* __restrict__ Pp, const __grid_constant__ WfSceneTable 
     const uint32_t n = ctr->shadow;
     const float offset = P.cfg.ray_offset;
     unsigned long long rays = 0;
-    auto fetch = [&](uint32_t i, Traversal<true, false, true>& tr, WfStack& stack) -> uint32_t {
+    auto fetch = [&](uint32_t i, Traversal<true, false, true, false>& tr, WfStack& stack) -> uint32_t {
         const float4 o = P.sh_o[i], d = P.sh_d[i];
         const uint32_t scene = __float_as_uint(o.w) >> kWfSlotBits;
         tr.start(vec3(o.x, o.y, o.z), vec3(d.x, d.y, d.z), offset, 1.0f - offset, scenes.v[scene].num_tris > 0, stack);
         return scene;
     };
-    auto finish = [&](uint32_t i, const Traversal<true, false, true>& tr) {
+    auto finish = [&](uint32_t i, const Traversal<true, false, true, false>& tr) {
         const uint32_t slot = __float_as_uint(P.sh_o[i].w) & kWfSlotMask;
         if (tr.hit < 0) {
             const float4 c = P.color[slot], a = P.sh_c[i];
