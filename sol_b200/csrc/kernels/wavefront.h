@@ -21,15 +21,21 @@ constexpr int kWfBins = 6;
 constexpr int kWfRefillBelow = SOL_WF_REFILL_BELOW;
 
 #ifndef SOL_WF_TRACE_MIN_BLOCKS
-#define SOL_WF_TRACE_MIN_BLOCKS 6
+#define SOL_WF_TRACE_MIN_BLOCKS 3
 #endif
 /// Resident 256-thread blocks per SM the traversal stages' registers must allow.
+/// 3 (up to 80 registers, nothing spilled): the stages are chains of dependent
+/// node fetches that spilling (6 blocks, 40 registers) lengthens, and every
+/// bounce launches the full grid, so fewer blocks also cost less where the
+/// queues are short.  24 views (about 25M paths) 9.86 ms at 6 blocks, 8.91 at
+/// 4, 8.73 at 3, 8.82 at 2; 4 small views 1.25, 1.06, 0.94 ms.
 constexpr int kWfTraceMinBlocks = SOL_WF_TRACE_MIN_BLOCKS;
 
 #ifndef SOL_WF_SHADE_MIN_BLOCKS
-#define SOL_WF_SHADE_MIN_BLOCKS 3
+#define SOL_WF_SHADE_MIN_BLOCKS 2
 #endif
-/// Resident 256-thread blocks per SM the shading stage's registers must allow.
+/// Resident 256-thread blocks per SM the shading stage's registers must allow
+/// (24 views with the above: 8.97 ms at 3, 8.78 at 2, 8.79 at 1).
 constexpr int kWfShadeMinBlocks = SOL_WF_SHADE_MIN_BLOCKS;
 
 #ifndef SOL_WF_SHADE_RESTART
