@@ -108,16 +108,7 @@ int render_into(SolGpuScene* scene, const SolGpuCamera* camera, const SolGpuConf
     cudaError_t e = cudaMemsetAsync(scene->counters, 0, sizeof(DeviceCounters), stream);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
     SceneView v = scene->view;
-    // The full-occupancy build for renders of many paths per resident lane,
-    // the 12-block build (fewer spills per path) for smaller ones.
     const bool basic = scene->basic_shading;
-    const int per_sm_full = megakernel_blocks_per_sm(scene->instrumented, true, basic);
-    if (per_sm_full <= 0) return fail(SOL_GPU_ERR_CUDA, "megakernel occupancy query failed");
-    const uint64_t paths = (uint64_t)width * height * sample_count;
-    const bool full = paths >= kMegakernelFullPathsPerLane * (uint64_t)per_sm_full * scene->num_sms * kMegakernelBlock;
-    const int per_sm = full ? per_sm_full : megakernel_blocks_per_sm(scene->instrumented, false, basic);
-    if (per_sm <= 0) return fail(SOL_GPU_ERR_CUDA, "megakernel occupancy query failed");
-    const int grid = per_sm * scene->num_sms;
     const DCamera cam = to_camera(*camera);
     // Split schedule (one work item per pixel sample, measured faster than the
     // per-pixel schedule on small and full-size frames alike) for every render
@@ -152,6 +143,16 @@ int render_into(SolGpuScene* scene, const SolGpuCamera* camera, const SolGpuConf
             return cuda_fail(e, "cudaMalloc split scratch");
         }
     }
+    // One path per work item (lean): the full-occupancy build when there is
+    // enough to trace for its resident lanes (kMegakernelFullVerticesPerLane).
+    const bool lean = split || sample_count == 1;
+    int per_sm = megakernel_blocks_per_sm(scene->instrumented, lean, true, basic);
+    const uint64_t vertices = pixels * (split ? chunk : 1) *
+        std::min(std::max(config->max_path_len, kMegakernelMinCountedLen), kMegakernelMaxCountedLen);
+    const bool full = vertices > kMegakernelFullVerticesPerLane * (uint64_t)per_sm * scene->num_sms * kMegakernelBlock;
+    if (lean && !full) per_sm = megakernel_blocks_per_sm(scene->instrumented, lean, false, basic);
+    if (per_sm <= 0) return fail(SOL_GPU_ERR_CUDA, "megakernel occupancy query failed");
+    const int grid = per_sm * scene->num_sms;
     cudaEventRecord(scene->ev_start, stream);
     if (split)
         e = launch_megakernel_split(v, cam, to_config(*config), sample_index, sample_count, width, height, film,

@@ -21,16 +21,12 @@ namespace sol_b200 {
 #define SOL_MEGAKERNEL_VIEWS_MIN_BLOCKS 12   // the multi-view megakernel: 40 registers (measured faster than 16 and 10)
 #endif
 #ifndef SOL_MEGAKERNEL_SMALL_MIN_BLOCKS
-#define SOL_MEGAKERNEL_SMALL_MIN_BLOCKS 12   // 40 registers: renders of a few paths per lane, where spills cost more
-#endif
-#ifndef SOL_MEGAKERNEL_SPLIT_LEAN
-#define SOL_MEGAKERNEL_SPLIT_LEAN 1   // 1: the split schedule's lean kernel (pt_megakernel_lean)
+#define SOL_MEGAKERNEL_SMALL_MIN_BLOCKS 6   // 80 registers, hardly any spills: renders that end with their longest paths
 #endif
 #ifndef SOL_LEAN_REGEN_MIN
-// The split schedule's lean kernel: idle lanes of a warp claim new work items
-// together once at least this many are idle (0: the warp claims only when all
-// 32 paths have ended).  Measured (frame / Cornell Mpaths/s): 0 -> 2455 /
-// 604, 8 -> 2593 / 654, 12 -> 2617 / 652, 16 -> 2635 / 645, 20 -> 2636 / 650,
+// The lean kernel: idle lanes of a warp claim new work items together once at
+// least this many of its 32 are idle.  Measured (frame / Cornell Mpaths/s):
+// 8 -> 2593 / 654, 12 -> 2617 / 652, 16 -> 2635 / 645, 20 -> 2636 / 650,
 // 24 -> 2636 / 648, 32 -> 2419 / 589.
 #define SOL_LEAN_REGEN_MIN 20
 #endif
@@ -43,9 +39,18 @@ constexpr int kMegakernelBlock = SOL_MEGAKERNEL_BLOCK;
 constexpr int kMegakernelMinBlocks = SOL_MEGAKERNEL_MIN_BLOCKS;
 constexpr int kMegakernelSmallMinBlocks = SOL_MEGAKERNEL_SMALL_MIN_BLOCKS;
 constexpr int kMegakernelViewsMinBlocks = SOL_MEGAKERNEL_VIEWS_MIN_BLOCKS;
-/// K1 renders with at least this many paths per resident lane of the
-/// full-occupancy build use it; smaller renders use the 12-block build.
-constexpr uint64_t kMegakernelFullPathsPerLane = 8;
+/// Renders use the full-occupancy build (kMegakernelMinBlocks) when they have
+/// more than this many path vertices to trace per resident lane of it, counting
+/// each path with its length limit, taken between the two bounds below (limits
+/// beyond 16 are cut short by the roulette).  Fewer paths than that are under
+/// way together from the start, and the launch lasts as long as its longest
+/// paths do, which the 6-block build, spilling hardly at all, traces sooner.
+/// Measured, 6 against 12 blocks (us): Cornell, limit 16: 25.6k paths x 4 278 /
+/// 348, 205k 394 / 403, 262k 496 / 483, 480k 755 / 700, 1M 1530 / 1353; sphere
+/// fields, limit 8: 230k 392 / 432, 410k 252 / 281, 518k 217 / 229, textured
+/// 240k 233 / 253; 1M triangles, 2M paths 1037 / 993, 8M 3281 / 2848.
+constexpr uint64_t kMegakernelFullVerticesPerLane = 16;
+constexpr uint32_t kMegakernelMinCountedLen = 8, kMegakernelMaxCountedLen = 16;
 constexpr int kTraceBlock = 64;
 #ifndef SOL_SPLIT_SCRATCH_MAX_MB
 #define SOL_SPLIT_SCRATCH_MAX_MB 2048
@@ -67,14 +72,16 @@ struct L2Window {
 };
 
 /// Resident blocks per SM of the megakernel (for sizing its persistent grid);
-/// `full`: the full-occupancy build (kMegakernelMinBlocks), else the
-/// kMegakernelSmallMinBlocks build; `basic`: the build without image textures
+/// `lean`: the kernel of one path per work item (the split schedule and single
+/// samples), in its full-occupancy build (`full`, kMegakernelMinBlocks) or the
+/// kMegakernelSmallMinBlocks one; `basic`: the build without image textures
 /// and Interp BSDFs, for scenes that have neither (SolGpuScene::basic_shading).
-int megakernel_blocks_per_sm(bool instrumented, bool full, bool basic);
+int megakernel_blocks_per_sm(bool instrumented, bool lean, bool full, bool basic);
 
 /// K1: renders samples [sample_index, sample_index + sample_count) of every
 /// pixel and adds each pixel's sum into `film` (3 planes of width*height).
-/// `counters` must be zeroed before the launch.
+/// A single sample goes to the lean kernel (`full` picks its build), several
+/// to the per-pixel schedule.  `counters` must be zeroed before the launch.
 cudaError_t launch_megakernel(const SceneView& s, const DCamera& cam, const DConfig& cfg,
                               uint64_t sample_index, uint32_t sample_count, uint32_t width, uint32_t height,
                               float* film, DeviceCounters* counters, bool instrumented, bool full, bool basic,

@@ -169,23 +169,24 @@ pt_megakernel(SceneView s, DCamera cam, DConfig cfg, uint64_t sample_index, uint
     }
 }
 
-/// K1 in the split schedule, lean form: every work item is one path, so a lane
-/// claims an item, traces its path to the end and writes the colour (0 +
-/// colour, as the per-pixel sum starts) to the scratch plane of its sample,
-/// then claims the next.  The same path computation and the same scratch as
-/// pt_megakernel<kCount = false, kSplit = true>, with less state live across
-/// the traversal (no per-pixel sum, sample range or loop bounds: the claim
-/// loop ends with the items and the bounce loop with the path length, and
-/// the traversal keeps its own step bound), so the register-capped builds
-/// spill less.  When the warp claims work is set by SOL_LEAN_REGEN_MIN: by
-/// default its idle lanes claim consecutive items together once 20 of its 32
-/// lanes are idle; with 0 the warp claims 32 items at once (one sample of one
-/// 8x4 tile) and waits for its longest path before the next claim.  Both beat
-/// regenerating each lane's path at once, which lets the lanes drift apart.
-template <int kMinBlocks, bool kBasic>
+/// K1, lean form: every work item is one path, so a lane claims an item, traces
+/// its path to the end and writes the colour, then claims the next.  In the
+/// split schedule (kFilm = false) the colour (0 + colour, as the per-pixel sum
+/// starts) goes to the scratch plane of its sample; with kFilm, for renders of
+/// a single sample, it is the pixel's sum and is added into the film
+/// (image.h:54-60).  The same path computation as pt_megakernel with less state
+/// live across the traversal (no per-pixel sum, sample range or loop bounds:
+/// the claim loop ends with the items and the bounce loop with the path
+/// length, and the traversal keeps its own step bound), so the register-capped
+/// builds spill less.  The warp's idle lanes claim consecutive items together
+/// once `regen` of them are idle (SOL_LEAN_REGEN_MIN of 32), which beats both
+/// waiting for the warp's longest path and regenerating each lane's path at
+/// once.  Only the first `lanes` lanes of a warp take paths (lanes_per_warp).
+template <int kMinBlocks, bool kBasic, bool kFilm>
 __global__ void __launch_bounds__(kMegakernelBlock, kMinBlocks)
 pt_megakernel_lean(SceneView s, DCamera cam, DConfig cfg, uint64_t sample_index, uint32_t sample_count,
-                   uint32_t width, uint32_t height, float* __restrict__ scratch, DeviceCounters* __restrict__ ctr) {
+                   uint32_t width, uint32_t height, float* __restrict__ scratch, DeviceCounters* __restrict__ ctr,
+                   uint32_t lanes, uint32_t regen) {
     const uint32_t tiles_x = (width + 7u) / 8u;
     const uint32_t total = tiles_x * ((height + 3u) / 4u) * 32u;   // items of one sample
     const uint32_t items = total * sample_count;
@@ -194,23 +195,21 @@ pt_megakernel_lean(SceneView s, DCamera cam, DConfig cfg, uint64_t sample_index,
     TraversalCounters tc{0u, 0u};
     uint32_t n_paths = 0, n_rays = 0, n_shadow = 0;
     LocalStack stack;
-#if SOL_LEAN_REGEN_MIN
     // One bounce per iteration; the warp's idle lanes claim new items together
-    // once at least SOL_LEAN_REGEN_MIN of them are idle (or no lane has a
-    // path), so lanes neither wait for the warp's longest path nor drift apart
+    // once at least `regen` of them are idle (or no lane has a path), so lanes neither wait for the warp's longest path nor drift apart
     // one by one.  Every lane stays in the loop until the whole warp is done
     // (the exit test is a warp-uniform vote), so the full-warp votes and the
     // barrier see all 32 lanes; every iteration either advances a live path by
     // one bounce or claims items, so the loop ends with the items.
     PathState ps;
     uint32_t k = 0, px = 0, py = 0;
-    bool alive = false, done = false;
+    bool alive = false, done = (threadIdx.x & 31u) >= lanes;
     while (true) {
         __syncwarp();
         const unsigned idle = __ballot_sync(0xffffffffu, !alive && !done);
         const unsigned busy = __ballot_sync(0xffffffffu, alive);
         if (busy == 0u && idle == 0u) break;
-        if (!alive && !done && (__popc(idle) >= SOL_LEAN_REGEN_MIN || busy == 0u)) {
+        if (!alive && !done && ((uint32_t)__popc(idle) >= regen || busy == 0u)) {
             const uint32_t item = claim_items(&ctr->next_item);
             if (item >= items) {
                 done = true;
@@ -254,54 +253,20 @@ pt_megakernel_lean(SceneView s, DCamera cam, DConfig cfg, uint64_t sample_index,
             }
             if (end) {
                 const Rgb c = rgb(0.0f) + ps.color;   // path_tracer.cpp:19; the sum pass adds in sample order
-                float* f = scratch + (size_t)k * 3u * plane + (size_t)py * width + px;
-                f[0] = c.r;
-                f[plane] = c.g;
-                f[2 * plane] = c.b;
+                float* f = scratch + (kFilm ? 0 : (size_t)k * 3u * plane) + (size_t)py * width + px;
+                if (kFilm) {
+                    f[0] += c.r;
+                    f[plane] += c.g;
+                    f[2 * plane] += c.b;
+                } else {
+                    f[0] = c.r;
+                    f[plane] = c.g;
+                    f[2 * plane] = c.b;
+                }
                 alive = false;
             }
         }
     }
-#else
-    while (true) {
-        const uint32_t item = claim_items(&ctr->next_item);
-        if (item >= items) break;
-        const uint32_t k = item / total;
-        const uint32_t it = item - k * total;
-        const uint32_t tile = it >> 5, l = it & 31u;
-        const uint32_t px = (tile % tiles_x) * 8u + (l & 7u);
-        const uint32_t py = (tile / tiles_x) * 4u + (l >> 3);
-        if (px >= width || py >= height) continue;   // padding of a partial tile
-        PathState ps;
-        start_path(ps, cam, sample_index + k, px, py, width, height);
-        ++n_paths;
-        while (ps.path_len < cfg.max_path_len) {
-            // closest hit (path_tracer.cpp:42)
-            float t = kFloatMax;
-            float hu, hv;
-            const int slot = traverse_closest_uv<false>(s, ps.org, ps.dir, ps.tmin, t, hu, hv, tc, stack);
-            ++n_rays;
-            if (slot < 0) break;
-            VertexOut vo;
-            shade_vertex<kBasic>(s, cfg, light_pick_prob, slot, t, ps, vo, true, hu, hv);
-            // shadow ray of this vertex (path_tracer.cpp:72-74)
-            if (vo.has_shadow) {
-                const bool occ =
-                    occluded<false>(s, vo.sh_org, vo.sh_dir, cfg.ray_offset, 1.0f - cfg.ray_offset, tc, stack);
-                ++n_rays;
-                ++n_shadow;
-                if (!occ) ps.color = ps.color + vo.pending;
-            }
-            if (vo.end) break;
-            ++ps.path_len;
-        }
-        const Rgb c = rgb(0.0f) + ps.color;   // path_tracer.cpp:19, the sum pass adds the rest in sample order
-        float* f = scratch + (size_t)k * 3u * plane + (size_t)py * width + px;
-        f[0] = c.r;
-        f[plane] = c.g;
-        f[2 * plane] = c.b;
-    }
-#endif
     __syncwarp();
     unsigned long long v0 = warp_sum_u64(n_paths), v1 = warp_sum_u64(n_rays), v2 = warp_sum_u64(n_shadow);
     if ((threadIdx.x & 31) == 0) {
@@ -489,33 +454,53 @@ sum_samples_views(const WfView* __restrict__ views, uint32_t num_views, uint64_t
 
 namespace {
 
-/// The K1 instantiation for a counting flag, schedule, occupancy target and
-/// shading (basic: the scene has no image textures and no Interp BSDFs; the
-/// counting build always has full shading).
+/// The K1 instantiation for a schedule, occupancy target and shading (basic:
+/// the scene has no image textures and no Interp BSDFs; the counting build
+/// always has full shading).
 template <bool kSplit>
-auto megakernel_fn(bool instrumented, bool full, bool basic) {
-    if (instrumented) return full ? pt_megakernel<true, kSplit, kMegakernelMinBlocks, false>
-                                  : pt_megakernel<true, kSplit, kMegakernelSmallMinBlocks, false>;
-#if SOL_MEGAKERNEL_SPLIT_LEAN
-    if (kSplit) {
-        if (basic) return full ? pt_megakernel_lean<kMegakernelMinBlocks, true>
-                               : pt_megakernel_lean<kMegakernelSmallMinBlocks, true>;
-        return full ? pt_megakernel_lean<kMegakernelMinBlocks, false>
-                    : pt_megakernel_lean<kMegakernelSmallMinBlocks, false>;
-    }
-#endif
-    if (basic) return full ? pt_megakernel<false, kSplit, kMegakernelMinBlocks, true>
-                           : pt_megakernel<false, kSplit, kMegakernelSmallMinBlocks, true>;
-    return full ? pt_megakernel<false, kSplit, kMegakernelMinBlocks, false>
-                : pt_megakernel<false, kSplit, kMegakernelSmallMinBlocks, false>;
+auto megakernel_fn(bool instrumented, bool basic) {
+    if (instrumented) return pt_megakernel<true, kSplit, kMegakernelMinBlocks, false>;
+    return basic ? pt_megakernel<false, kSplit, kMegakernelMinBlocks, true>
+                 : pt_megakernel<false, kSplit, kMegakernelMinBlocks, false>;
+}
+template <bool kFilm>
+auto lean_fn(bool full, bool basic) {
+    if (basic) return full ? pt_megakernel_lean<kMegakernelMinBlocks, true, kFilm>
+                           : pt_megakernel_lean<kMegakernelSmallMinBlocks, true, kFilm>;
+    return full ? pt_megakernel_lean<kMegakernelMinBlocks, false, kFilm>
+                : pt_megakernel_lean<kMegakernelSmallMinBlocks, false, kFilm>;
+}
+
+/// Lanes of each warp that take paths: all 32 unless the launch's warps could
+/// give every path a lane with fewer (a power of two).  Paths that share a
+/// warp wait for each other's divergent branches, so a render of a few
+/// thousand paths is done sooner spread over all resident warps: 64x48 Cornell
+/// preview 210 -> 128 us (one lane), 128x128 184 -> 165 (8), 200x120 textured
+/// 157 -> 126 (8).
+uint32_t lanes_per_warp(uint64_t paths, int grid) {
+    const uint64_t warps = (uint64_t)grid * (kMegakernelBlock / 32);
+    uint32_t lanes = 1;
+    while (lanes < 32u && lanes * warps < paths) lanes *= 2;
+    return lanes;
+}
+
+template <bool kFilm>
+cudaError_t launch_lean(const SceneView& s, const DCamera& cam, const DConfig& cfg, uint64_t sample_index,
+                        uint32_t sample_count, uint32_t width, uint32_t height, float* out, DeviceCounters* counters,
+                        bool full, bool basic, int grid, cudaStream_t stream, const L2Window& l2) {
+    const uint32_t lanes = lanes_per_warp((uint64_t)width * height * sample_count, grid);
+    const uint32_t regen = std::max(1u, lanes * (uint32_t)SOL_LEAN_REGEN_MIN / 32u);
+    return launch_l2(lean_fn<kFilm>(full, basic), grid, kMegakernelBlock, 0, stream, l2, s, cam, cfg, sample_index,
+                     sample_count, width, height, out, counters, lanes, regen);
 }
 
 }  // namespace
 
-int megakernel_blocks_per_sm(bool instrumented, bool full, bool basic) {
+int megakernel_blocks_per_sm(bool instrumented, bool lean, bool full, bool basic) {
     int n = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, megakernel_fn<true>(instrumented, full, basic),
-                                                                  kMegakernelBlock, 0);
+    const cudaError_t e = lean && !instrumented
+        ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, lean_fn<false>(full, basic), kMegakernelBlock, 0)
+        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, megakernel_fn<true>(instrumented, basic), kMegakernelBlock, 0);
     return e == cudaSuccess ? n : -1;
 }
 
@@ -523,7 +508,9 @@ cudaError_t launch_megakernel(const SceneView& s, const DCamera& cam, const DCon
                               uint64_t sample_index, uint32_t sample_count, uint32_t width, uint32_t height,
                               float* film, DeviceCounters* counters, bool instrumented, bool full, bool basic,
                               int grid, cudaStream_t stream, const L2Window& l2) {
-    return launch_l2(megakernel_fn<false>(instrumented, full, basic), grid, kMegakernelBlock, 0, stream, l2, s, cam, cfg,
+    if (!instrumented && sample_count == 1)
+        return launch_lean<true>(s, cam, cfg, sample_index, 1, width, height, film, counters, full, basic, grid, stream, l2);
+    return launch_l2(megakernel_fn<false>(instrumented, basic), grid, kMegakernelBlock, 0, stream, l2, s, cam, cfg,
                      sample_index, sample_count, width, height, film, counters);
 }
 
@@ -570,8 +557,10 @@ cudaError_t launch_megakernel_split(const SceneView& s, const DCamera& cam, cons
         cudaError_t e = cudaSuccess;
         if (c0 > 0) e = cudaMemsetAsync(&counters->next_item, 0, sizeof(counters->next_item), stream);
         if (e != cudaSuccess) return e;
-        e = launch_l2(megakernel_fn<true>(instrumented, full, basic), grid, kMegakernelBlock, 0, stream, l2, s, cam, cfg,
-                      sample_index + c0, k, width, height, scratch, counters);
+        e = instrumented ? launch_l2(megakernel_fn<true>(true, basic), grid, kMegakernelBlock, 0, stream, l2, s, cam, cfg,
+                                     sample_index + c0, k, width, height, scratch, counters)
+                         : launch_lean<false>(s, cam, cfg, sample_index + c0, k, width, height, scratch, counters, full,
+                                              basic, grid, stream, l2);
         if (e != cudaSuccess) return e;
         sum_samples<<<blocks, 256, 0, stream>>>(scratch, k, plane, running, c0 == 0, c0 + k == sample_count, film);
         e = cudaGetLastError();
