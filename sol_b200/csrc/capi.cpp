@@ -83,9 +83,8 @@ cudaError_t upload(T** dst, const std::vector<T>& src) {
 void release(SolGpuScene* s) {
     if (!s) return;
     DeviceGuard g(s->device);
-    cudaFree(s->boxes); cudaFree(s->tris); cudaFree(s->shade); cudaFree(s->bsdfs);
-    cudaFree(s->textures); cudaFree(s->images); cudaFree(s->texels); cudaFree(s->lights);
-    cudaFree(s->counters); cudaFree(s->film_tmp); cudaFree(s->split_scratch); cudaFree(s->adj_texels4); cudaFree(s->param_offsets); cudaFree(s->fault);
+    cudaFree(s->boxes); cudaFree(s->tris); cudaFree(s->shade); cudaFree(s->tables); cudaFree(s->texels);
+    cudaFree(s->film_tmp); cudaFree(s->split_scratch); cudaFree(s->adj_texels4);
     if (s->film_host) cudaFreeHost(s->film_host);
     if (s->ev_start) cudaEventDestroy(s->ev_start);
     if (s->ev_stop) cudaEventDestroy(s->ev_stop);
@@ -206,36 +205,42 @@ int sol_gpu_scene_create_ex(const SolGpuSceneDesc* desc, int device, uint32_t fl
     if (e == cudaSuccess) e = cudaEventCreate(&s->ev_start);
     if (e == cudaSuccess) e = cudaEventCreate(&s->ev_stop);
     float gpu_build_ms = 0.0f;
+    size_t num_nodes = flat.nodes.size();
     if (gpu_bvh && e == cudaSuccess) {
         // Build the hierarchy on the device from the mesh arrays.
         const uint32_t nv = desc->num_vertices, nt = desc->num_triangles;
-        float *d_v = nullptr, *d_n = nullptr, *d_uv = nullptr;
-        uint32_t* d_i = nullptr;
-        int32_t *d_b = nullptr, *d_l = nullptr;
-        auto up = [&](void** dst, const void* src, size_t bytes) {
-            if (e != cudaSuccess) return;
-            e = cudaMalloc(dst, bytes ? bytes : 1);
-            if (e == cudaSuccess && bytes) e = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
+        char* mesh = nullptr;   // the mesh arrays, one after another
+        size_t mesh_bytes = 0;
+        auto place = [&](size_t bytes) { const size_t at = mesh_bytes; mesh_bytes += (bytes + 255) & ~(size_t)255; return at; };
+        const size_t at_v = place(sizeof(float) * 3 * nv), at_n = place(sizeof(float) * 3 * nv);
+        const size_t at_uv = place(sizeof(float) * 2 * nv), at_i = place(sizeof(uint32_t) * 3 * nt);
+        const size_t at_b = place(sizeof(int32_t) * nt), at_l = place(sizeof(int32_t) * nt);
+        auto up = [&](size_t at, const void* src, size_t bytes) {
+            if (e == cudaSuccess && bytes) e = cudaMemcpy(mesh + at, src, bytes, cudaMemcpyHostToDevice);
         };
         cudaEvent_t b0, b1;
         cudaEventCreate(&b0);
         cudaEventCreate(&b1);
         cudaEventRecord(b0, s->stream);
-        up(reinterpret_cast<void**>(&d_v), desc->vertices, sizeof(float) * 3 * nv);
-        up(reinterpret_cast<void**>(&d_n), desc->normals, sizeof(float) * 3 * nv);
-        up(reinterpret_cast<void**>(&d_uv), desc->tex_coords, sizeof(float) * 2 * nv);
-        up(reinterpret_cast<void**>(&d_i), desc->indices, sizeof(uint32_t) * 3 * nt);
-        up(reinterpret_cast<void**>(&d_b), desc->tri_bsdf, sizeof(int32_t) * nt);
-        up(reinterpret_cast<void**>(&d_l), desc->tri_light, sizeof(int32_t) * nt);
+        e = cudaMalloc(reinterpret_cast<void**>(&mesh), mesh_bytes);
+        up(at_v, desc->vertices, sizeof(float) * 3 * nv);
+        up(at_n, desc->normals, sizeof(float) * 3 * nv);
+        up(at_uv, desc->tex_coords, sizeof(float) * 2 * nv);
+        up(at_i, desc->indices, sizeof(uint32_t) * 3 * nt);
+        up(at_b, desc->tri_bsdf, sizeof(int32_t) * nt);
+        up(at_l, desc->tri_light, sizeof(int32_t) * nt);
         if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);   // the build's stream does not wait for the copies
         LbvhResult r;
-        if (e == cudaSuccess) e = build_lbvh(d_v, d_i, d_n, d_uv, d_b, d_l, nt, s->stream, &r);
+        if (e == cudaSuccess)
+            e = build_lbvh(reinterpret_cast<float*>(mesh + at_v), reinterpret_cast<uint32_t*>(mesh + at_i),
+                           reinterpret_cast<float*>(mesh + at_n), reinterpret_cast<float*>(mesh + at_uv),
+                           reinterpret_cast<int32_t*>(mesh + at_b), reinterpret_cast<int32_t*>(mesh + at_l), nt, s->stream, &r);
         cudaEventRecord(b1, s->stream);
         cudaEventSynchronize(b1);
         cudaEventElapsedTime(&gpu_build_ms, b0, b1);
         cudaEventDestroy(b0);
         cudaEventDestroy(b1);
-        cudaFree(d_v); cudaFree(d_n); cudaFree(d_uv); cudaFree(d_i); cudaFree(d_b); cudaFree(d_l);
+        cudaFree(mesh);
         if (e == cudaSuccess) {
             s->boxes = r.boxes;
             s->nodes = r.nodes;
@@ -244,7 +249,7 @@ int sol_gpu_scene_create_ex(const SolGpuSceneDesc* desc, int device, uint32_t fl
             flat.depth = r.depth;
             flat.sah_cost = r.sah_cost;
             flat.top_nodes = 0;
-            flat.nodes.assign(r.num_nodes, DNode{});   // sizes only: the arrays are already on the device
+            num_nodes = r.num_nodes;
             if (r.depth > (uint32_t)kTraversalStack) {
                 release(s);
                 return fail(SOL_GPU_ERR_UNSUPPORTED, "GPU BVH depth " + std::to_string(r.depth) +
@@ -265,14 +270,7 @@ int sol_gpu_scene_create_ex(const SolGpuSceneDesc* desc, int device, uint32_t fl
         if (e == cudaSuccess) e = upload(&s->tris, flat.tris);
         if (e == cudaSuccess) e = upload(&s->shade, flat.shade);
     }
-    if (e == cudaSuccess) e = upload(&s->bsdfs, flat.bsdfs);
-    if (e == cudaSuccess) e = upload(&s->textures, flat.textures);
-    if (e == cudaSuccess) e = upload(&s->images, flat.images);
     if (e == cudaSuccess) e = upload(&s->texels, flat.texels);
-    if (e == cudaSuccess) e = upload(&s->lights, flat.lights);
-    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&s->counters), sizeof(DeviceCounters));
-    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&s->fault), sizeof(unsigned int));
-    if (e == cudaSuccess) e = cudaMemset(s->fault, 0, sizeof(unsigned int));
     // Parameter layout: constants in texture order, then the images' texel blocks.
     s->host_textures = flat.textures;
     s->host_images = flat.images;
@@ -290,9 +288,32 @@ int sol_gpu_scene_create_ex(const SolGpuSceneDesc* desc, int device, uint32_t fl
     s->param_count = off;
     for (size_t i = 0; i < flat.textures.size(); ++i)
         if (flat.textures[i].kind == SOL_GPU_TEX_IMAGE) s->texture_offsets[i] = s->image_offsets[flat.textures[i].image];
+    // The small tables, the counters and the fault word (both zero) in one
+    // allocation and one copy.
     {
-        std::vector<unsigned long long> offs(s->texture_offsets.begin(), s->texture_offsets.end());
-        if (e == cudaSuccess) e = upload(&s->param_offsets, offs);
+        const std::vector<unsigned long long> offs(s->texture_offsets.begin(), s->texture_offsets.end());
+        std::vector<char> image;
+        auto place = [&](const void* src, size_t bytes) {
+            const size_t at = image.size();
+            image.resize(at + ((std::max<size_t>(bytes, 1) + 255) & ~(size_t)255), 0);
+            if (src && bytes) std::memcpy(image.data() + at, src, bytes);
+            return at;
+        };
+        auto table = [&](const auto& v) { return place(v.data(), v.size() * sizeof(v[0])); };
+        const size_t bsdfs = table(flat.bsdfs), textures = table(flat.textures), images = table(flat.images);
+        const size_t lights = table(flat.lights), offsets = table(offs);
+        const size_t counters = place(nullptr, sizeof(DeviceCounters)), fault = place(nullptr, sizeof(unsigned int));
+        if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&s->tables), image.size());
+        if (e == cudaSuccess) e = cudaMemcpy(s->tables, image.data(), image.size(), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) {
+            s->bsdfs = reinterpret_cast<DBsdf*>(s->tables + bsdfs);
+            s->textures = reinterpret_cast<DTexture*>(s->tables + textures);
+            s->images = reinterpret_cast<DImage*>(s->tables + images);
+            s->lights = reinterpret_cast<DLight*>(s->tables + lights);
+            s->param_offsets = reinterpret_cast<unsigned long long*>(s->tables + offsets);
+            s->counters = reinterpret_cast<DeviceCounters*>(s->tables + counters);
+            s->fault = reinterpret_cast<unsigned int*>(s->tables + fault);
+        }
     }
     // The uploads (and the box nodes made from them) are on the legacy stream, renders on any.
     if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
@@ -309,9 +330,9 @@ int sol_gpu_scene_create_ex(const SolGpuSceneDesc* desc, int device, uint32_t fl
     s->view.num_lights = (uint32_t)flat.lights.size();
     s->view.num_tris = desc->num_triangles;
     s->view.param_offsets = s->param_offsets;
-    s->view.num_nodes = (uint32_t)flat.nodes.size();
+    s->view.num_nodes = (uint32_t)num_nodes;
     const size_t num_tris = gpu_bvh ? desc->num_triangles : flat.tris.size();
-    s->default_max_steps = (uint32_t)std::min<uint64_t>(2ull * (flat.nodes.size() + num_tris) + 16ull, 0xffffffffull);
+    s->default_max_steps = (uint32_t)std::min<uint64_t>(2ull * (num_nodes + num_tris) + 16ull, 0xffffffffull);
     s->view.max_steps = s->default_max_steps;
     s->view.fault = s->fault;
     s->basic_shading =
@@ -320,10 +341,10 @@ int sol_gpu_scene_create_ex(const SolGpuSceneDesc* desc, int device, uint32_t fl
         std::none_of(flat.bsdfs.begin(), flat.bsdfs.end(), [](const DBsdf& b) { return b.kind == SOL_GPU_BSDF_INTERP; });
 
     s->info.num_triangles = desc->num_triangles;
-    s->info.num_nodes = (uint32_t)flat.nodes.size();
+    s->info.num_nodes = (uint32_t)num_nodes;
     s->info.bvh_depth = flat.depth;
     s->info.sah_cost = flat.sah_cost;
-    s->info.device_bytes = flat.nodes.size() * (sizeof(DBoxNode) + sizeof(DNode)) + num_tris * (sizeof(DTri) + sizeof(DTriShade));
+    s->info.device_bytes = num_nodes * (sizeof(DBoxNode) + sizeof(DNode)) + num_tris * (sizeof(DTri) + sizeof(DTriShade));
     s->info.build_ms = (float)flat.build_ms + gpu_build_ms;
 #if SOL_L2_PERSIST
     // Keep the upper BVH levels (stored first) in L2: raise this process's

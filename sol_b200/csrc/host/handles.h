@@ -19,6 +19,7 @@ struct SolGpuScene {
     sol_b200::DNode* nodes = nullptr;      // the second half of `boxes`
     sol_b200::DTri* tris = nullptr;
     sol_b200::DTriShade* shade = nullptr;
+    char* tables = nullptr;          // one allocation: bsdfs, textures, images, lights, param_offsets, counters, fault
     sol_b200::DBsdf* bsdfs = nullptr;
     sol_b200::DTexture* textures = nullptr;
     sol_b200::DImage* images = nullptr;
