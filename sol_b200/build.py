@@ -24,7 +24,7 @@ LIB = LIB_DIR / "libsol_gpu.so"
 PROBE_LIB = LIB_DIR / "libsol_probe.so"   # memory probes for the roofline (bench only)
 
 CUDA_SOURCES = ["kernels/megakernel.cu", "kernels/trace.cu", "kernels/wavefront.cu", "kernels/adjoint.cu",
-                "kernels/lbvh.cu", "noalloc.cu"]
+                "kernels/adjoint_small.cu", "kernels/lbvh.cu", "noalloc.cu"]
 HOST_SOURCES = ["capi.cpp", "batch.cpp", "job.cpp", "host/flatten.cpp"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

@@ -645,7 +645,7 @@ int sol_gpu_batch_forward_adjoint(SolGpuBatch* b, const SolGpuConfig* config, co
     if (guard.err != cudaSuccess) return cuda_fail(guard.err, "cudaSetDevice");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     std::vector<AdjView> v(n);
-    uint64_t items = 0;
+    uint64_t items = 0, paths = 0;
     for (uint32_t i = 0; i < n; ++i) {
         const SolGpuAdjointView& a = views[i];
         if (a.view.scene >= b->scenes.size()) return fail(SOL_GPU_ERR_INVALID_ARG, "view scene index out of range");
@@ -666,6 +666,7 @@ int sol_gpu_batch_forward_adjoint(SolGpuBatch* b, const SolGpuConfig* config, co
         w.item_begin = (uint32_t)items;
         w.group = fused_group(a.view.sample_count);
         items += fused_items(a.view.width, a.view.height, a.view.sample_count);
+        paths += (uint64_t)a.view.width * a.view.height * a.view.sample_count;
         if (items > 0xffffffffull) return fail(SOL_GPU_ERR_INVALID_ARG, "batch too large");
     }
     cudaError_t e = cudaSuccess;
@@ -684,12 +685,13 @@ int sol_gpu_batch_forward_adjoint(SolGpuBatch* b, const SolGpuConfig* config, co
     if (n > 0) e = cudaMemcpyAsync(b->d_adj_views, v.data(), sizeof(AdjView) * n, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->d_dc, 0, sizeof(DeviceCounters), st);
     if (e != cudaSuccess) return cuda_fail(e, "fused batch upload");
-    const int per_sm = fused_blocks_per_sm();
+    const AdjointBuild build = adjoint_build(paths, config->max_path_len, b->num_sms);
+    const int per_sm = fused_blocks_per_sm(build);
     if (per_sm <= 0) return fail(SOL_GPU_ERR_CUDA, "fused kernel occupancy query failed");
     cudaEventRecord(b->ev_start, st);
     if (n > 0) {
         e = launch_fused_forward_adjoint(b->d_adj_views, n, (uint32_t)items, b->d_scenes, to_config(*config),
-                                         b->d_dc, per_sm * b->num_sms, st);
+                                         b->d_dc, build, per_sm * b->num_sms, st);
         if (e != cudaSuccess) return cuda_fail(e, "fused forward/adjoint launch");
     }
     cudaEventRecord(b->ev_stop, st);

@@ -575,7 +575,8 @@ int sol_gpu_adjoint(SolGpuScene* scene, const SolGpuCamera* camera, const SolGpu
     cudaError_t e = cudaMemsetAsync(scene->counters, 0, sizeof(DeviceCounters), st);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
     const uint32_t n_shared = (uint32_t)std::min<uint64_t>(scene->constants_count, kAdjointMaxSharedParams);
-    const int per_sm = adjoint_blocks_per_sm(n_shared);
+    const AdjointBuild build = adjoint_build((uint64_t)width * height * sample_count, config->max_path_len, scene->num_sms);
+    const int per_sm = adjoint_blocks_per_sm(build, n_shared);
     if (per_sm <= 0) return fail(SOL_GPU_ERR_CUDA, "adjoint occupancy query failed");
     // Spread a pixel's samples over several lanes when the image alone would
     // not give every resident lane a few items.
@@ -601,7 +602,7 @@ int sol_gpu_adjoint(SolGpuScene* scene, const SolGpuCamera* camera, const SolGpu
     e = launch_adjoint(scene->view, to_camera(*camera), to_config(*config), sample_index, sample_count, chunk, width,
                        height, dl_dfilm, grad, n_shared, scene->adj_texels4, num_texels,
                        (uint32_t)scene->host_images.size(), scene->constants_count, scene->counters,
-                       per_sm * scene->num_sms, st);
+                       build, per_sm * scene->num_sms, st);
     if (e != cudaSuccess) return cuda_fail(e, "adjoint launch");
     cudaEventRecord(scene->ev_stop, st);
     scene->rendered = true;

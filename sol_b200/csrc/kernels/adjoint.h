@@ -8,11 +8,25 @@
 
 namespace sol_b200 {
 
-#ifndef SOL_ADJOINT_MIN_BLOCKS
-#define SOL_ADJOINT_MIN_BLOCKS 16  // resident blocks per SM the register allocation must allow (32 registers; measured fastest)
-#endif
 constexpr int kAdjointBlock = 128;
-constexpr int kAdjointMinBlocks = SOL_ADJOINT_MIN_BLOCKS;
+
+/// Builds of the adjoint kernels, by the resident blocks per SM their registers
+/// allow.  Records and shading leave little for the traversal at 16 blocks (32
+/// registers): a path then takes three times as long as at 4 (128 registers,
+/// hardly any spills), which only many paths in flight make up for.  So the
+/// build follows the path vertices of the call, counting each path with its
+/// length limit, per resident lane of the 4-block build.  Measured, adjoint at
+/// 4 / 8 / 16 blocks (us): textured Cornell, limit 16: 65.5k paths 488 / 597 /
+/// 905, 131k 903 / 737 / 1031, 262k 2140 / 1412 / 1299, 1.6M 17045 / 13023 /
+/// 10661; textured sphere field, limit 8: 33k 195 / 299 / 553, 131k 211 / 305 /
+/// 538, 262k 303 / 390 / 595.  Fused at 4 / 10 / 16 blocks: Cornell 65.5k 496 /
+/// 706 / 934, 262k 1834 / 1393 / 1357, 1M 7329 / 5293 / 5159; spheres 65.5k 202 /
+/// 380 / 536, 1M 945 / 865 / 1005, 2.2M 2276 / 1823 / 1860.
+enum class AdjointBuild { kSmall, kMiddle, kFull };
+constexpr int kAdjointSmallBlocks = 4, kAdjointMiddleBlocks = 8, kAdjointFullBlocks = 16;
+constexpr int kFusedFullBlocks = 10;   // the fused kernel's build for middle and full calls
+constexpr uint64_t kAdjointSmallVerticesPerLane = 20, kAdjointMiddleVerticesPerLane = 42;
+
 /// Longest path the adjoint replays (vertex records per lane).
 constexpr int kAdjointMaxDepth = 16;
 
@@ -48,13 +62,25 @@ inline uint64_t fused_items(uint32_t width, uint32_t height, uint32_t spp) {
 /// Most constant-texture values whose gradients a block gathers in shared memory.
 constexpr uint32_t kAdjointMaxSharedParams = 2048;   // 8 KB per block, so 16 blocks fit an SM
 
-int adjoint_blocks_per_sm(uint32_t n_shared);
-int fused_blocks_per_sm();
+/// The build for a call of `paths` paths of at most `max_path_len` vertices.
+AdjointBuild adjoint_build(uint64_t paths, uint32_t max_path_len, int sms);
+int adjoint_blocks_per_sm(AdjointBuild build, uint32_t n_shared);
+int fused_blocks_per_sm(AdjointBuild build);
+
+/// The kernels of each build (adjoint.cu, adjoint_small.cu).
+using AdjointFn = void (*)(SceneView, DCamera, DConfig, uint64_t, uint32_t, uint32_t, uint32_t, uint32_t, const float*,
+                           float*, uint32_t, float4*, DeviceCounters*, uint32_t);
+using FusedFn = void (*)(const AdjView*, uint32_t, uint32_t, const SceneView*, DConfig, DeviceCounters*);
+AdjointFn adjoint_fn_small();
+AdjointFn adjoint_fn_middle();
+AdjointFn adjoint_fn_full();
+FusedFn fused_fn_small();
+FusedFn fused_fn_full();
 
 /// Forward render + L2-loss adjoint of every view in one persistent launch.
 cudaError_t launch_fused_forward_adjoint(const AdjView* views, uint32_t num_views, uint32_t total_items,
-                                         const SceneView* scenes, const DConfig& cfg, DeviceCounters* counters, int grid,
-                                         cudaStream_t stream);
+                                         const SceneView* scenes, const DConfig& cfg, DeviceCounters* counters,
+                                         AdjointBuild build, int grid, cudaStream_t stream);
 
 /// Adds dL/d(parameters) of the paths of samples [sample_index, + sample_count)
 /// of every pixel into `grad`, given dL/dfilm (3 planes of width*height).  Each
@@ -67,8 +93,8 @@ cudaError_t launch_fused_forward_adjoint(const AdjView* views, uint32_t num_view
 cudaError_t launch_adjoint(const SceneView& s, const DCamera& cam, const DConfig& cfg, uint64_t sample_index,
                            uint32_t sample_count, uint32_t chunk, uint32_t width, uint32_t height,
                            const float* dl_dfilm, float* grad, uint32_t n_shared, float4* texels4, uint64_t num_texels,
-                           uint32_t num_images, uint64_t first_texel_param, DeviceCounters* counters, int grid,
-                           cudaStream_t stream);
+                           uint32_t num_images, uint64_t first_texel_param, DeviceCounters* counters,
+                           AdjointBuild build, int grid, cudaStream_t stream);
 
 /// Adds sum (scale * film - target)^2 into *loss and writes dL/dfilm (optional).
 cudaError_t launch_l2_loss(const float* film, const float* target, uint64_t n, float scale, float* dl_dfilm,

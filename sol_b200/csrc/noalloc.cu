@@ -144,7 +144,7 @@ extern "C" int sol_gpu_batch_forward_adjoint_noalloc(SolGpuScene* const* scenes,
     std::memset(image + kCountersOffset, 0, sizeof(DeviceCounters));
     SceneView* scene_table = reinterpret_cast<SceneView*>(image + kScenesOffset);
     AdjView* view_table = reinterpret_cast<AdjView*>(image + kViewsOffset);
-    uint64_t items = 0;
+    uint64_t items = 0, paths = 0;
     for (uint32_t i = 0; i < num_scenes; ++i) scene_table[i] = scenes[i]->view;
     for (uint32_t i = 0; i < num_views; ++i) {
         const SolGpuAdjointView& a = views[i];
@@ -166,6 +166,7 @@ extern "C" int sol_gpu_batch_forward_adjoint_noalloc(SolGpuScene* const* scenes,
         w.item_begin = (uint32_t)items;
         w.group = fused_group(a.view.sample_count);
         items += fused_items(a.view.width, a.view.height, a.view.sample_count);
+        paths += (uint64_t)a.view.width * a.view.height * a.view.sample_count;
         if (items > 0xffffffffull) return fail(SOL_GPU_ERR_INVALID_ARG, "batch too large");
     }
     DeviceGuard guard(device);
@@ -185,9 +186,10 @@ extern "C" int sol_gpu_batch_forward_adjoint_noalloc(SolGpuScene* const* scenes,
     int num_sms = 0;
     e = cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device);
     if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceGetAttribute");
-    const int per_sm = fused_blocks_per_sm();
+    const AdjointBuild build = adjoint_build(paths, config->max_path_len, num_sms);
+    const int per_sm = fused_blocks_per_sm(build);
     if (per_sm <= 0) return fail(SOL_GPU_ERR_CUDA, "fused kernel occupancy query failed");
     e = launch_fused_forward_adjoint(d_views, num_views, (uint32_t)items, d_scenes, to_config(*config), d_ctr,
-                                     per_sm * num_sms, st);
+                                     build, per_sm * num_sms, st);
     return e == cudaSuccess ? SOL_GPU_OK : cuda_fail(e, "fused forward/adjoint launch");
 }
