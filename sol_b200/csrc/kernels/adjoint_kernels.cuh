@@ -97,22 +97,29 @@ struct GradSink {
     float4* texels4;   // when set: image-texel gradients as (r, g, b, 0) per texel, gathered afterwards
 };
 
-/// Sums `v` over the lanes of the warp that pass the same `addr` and returns
-/// the sum on the lowest such lane (rank 0), 0 elsewhere.
-template <typename T>
-__device__ __forceinline__ T reduce_by_address(const void* addr, T v, bool& leader) {
+/// Sums `v` over the active lanes of the warp that pass the same `key`: the sums
+/// are on the lowest such lane, for which it returns true.  Every round, each
+/// lane that still holds a partial sum adds the next such lane's above it, and
+/// every other one drops out (after Westphal's warp-aggregated reduction), so
+/// one match and at most five rounds serve all values at once.
+template <typename T, int N>
+__device__ __forceinline__ bool reduce_by_key(unsigned long long key, T (&v)[N]) {
     const unsigned active = __activemask();
-    const unsigned peers = __match_any_sync(active, (unsigned long long)addr);
-    const int n = __popc(peers);
-    const int rank = __popc(peers & ((1u << lane()) - 1u));
-    T sum = v;
-    for (int s = 1; s < n; s <<= 1) {
-        const int src = rank + s < n ? (int)__fns(peers, 0, rank + s + 1) : (int)lane();
-        const T other = __shfl_sync(peers, sum, src);
-        if (rank + s < n && (rank & (2 * s - 1)) == 0) sum += other;
+    const unsigned same = __match_any_sync(active, key);
+    unsigned above = same & (0xfffffffeu << lane());
+    const int first = __ffs(same) - 1;
+    unsigned rank = __popc(same & ((1u << lane()) - 1u));
+    while (__any_sync(active, above != 0u)) {
+        const int next = __ffs(above);   // 0: none
+#pragma unroll
+        for (int c = 0; c < N; ++c) {
+            const T other = __shfl_sync(active, v[c], next ? next - 1 : (int)lane());
+            if (next) v[c] += other;
+        }
+        above &= __ballot_sync(active, !(rank & 1u));   // odd ranks were taken
+        rank >>= 1;
     }
-    leader = rank == 0;
-    return sum;
+    return (int)lane() == first;
 }
 
 #ifndef SOL_ADJOINT_NOINLINE
@@ -142,18 +149,23 @@ __device__ __forceinline__ T reduce_by_address(const void* addr, T v, bool& lead
 /// are summed first, otherwise every lane issues its own reduction.
 __device__ __forceinline__ void atomic_add_texel(const GradSink& g, uint64_t idx, float v);
 
-/// Adds `v` into parameter `idx`, after summing over the lanes that add into the same one.
-__device__ __forceinline__ void atomic_add_reduced(const GradSink& g, uint64_t idx, float v) {
-    bool leader;
-    const float sum = reduce_by_address(g.global + idx, v, leader);
-    if (!leader || sum == 0.0f) return;
-    if (idx < g.n_shared) atomicAdd(g.shared + idx, sum);
-    else atomicAdd(g.global + idx, sum);
+/// Adds v[0..N) into parameters idx, idx + 1, ... after summing over the lanes
+/// that add into the same ones.
+template <int N>
+__device__ __forceinline__ void atomic_add_reduced(const GradSink& g, uint64_t idx, float (&v)[N]) {
+    if (!reduce_by_key((unsigned long long)(g.global + idx), v)) return;
+#pragma unroll
+    for (int c = 0; c < N; ++c) {
+        if (v[c] == 0.0f) continue;
+        if (idx + c < g.n_shared) atomicAdd(g.shared + idx + c, v[c]);
+        else atomicAdd(g.global + idx + c, v[c]);
+    }
 }
 
 __device__ __forceinline__ void atomic_add_texel(const GradSink& g, uint64_t idx, float v) {
 #if SOL_ADJOINT_REDUCE_TEXELS
-    atomic_add_reduced(g, idx, v);
+    float one[1] = {v};
+    atomic_add_reduced(g, idx, one);
 #else
     if (v != 0.0f) atomicAdd(g.global + idx, v);
 #endif
@@ -165,9 +177,8 @@ __device__ SOL_ADJ_OUTLINE void scatter_color(const SceneView& s, const GradSink
     const DTexture t = s.textures[tex];
     const uint64_t base = s.param_offsets[tex];
     if (t.kind == SOL_GPU_TEX_CONSTANT_COLOR) {
-        atomic_add_reduced(grad, base + 0, a.r);
-        atomic_add_reduced(grad, base + 1, a.g);
-        atomic_add_reduced(grad, base + 2, a.b);
+        float v[3] = {a.r, a.g, a.b};
+        atomic_add_reduced(grad, base, v);
         return;
     }
     if (t.kind != SOL_GPU_TEX_IMAGE) return;
@@ -226,7 +237,8 @@ __device__ void scatter_scalar(const SceneView& s, const GradSink& grad, int tex
     if (tex < 0 || a == 0.0f) return;
     const DTexture t = s.textures[tex];
     if (t.kind == SOL_GPU_TEX_CONSTANT) {
-        atomic_add_reduced(grad, s.param_offsets[tex], a);
+        float v[1] = {a};
+        atomic_add_reduced(grad, s.param_offsets[tex], v);
         return;
     }
     scatter_color(s, grad, tex, uv, rgb(0.2126f * a, 0.7152f * a, 0.0722f * a));
@@ -625,10 +637,8 @@ fused_forward_adjoint(const AdjView* __restrict__ views, uint32_t num_views, uin
                 V.film[i] += sum.r;
                 V.film[i + plane] += sum.g;
                 V.film[i + 2 * plane] += sum.b;
-                bool first_lane;
-                const double l2 = reduce_by_address(V.loss, (double)d.r * d.r + (double)d.g * d.g + (double)d.b * d.b,
-                                                    first_lane);
-                if (first_lane) atomicAdd(V.loss, l2);
+                double l2[1] = {(double)d.r * d.r + (double)d.g * d.g + (double)d.b * d.b};
+                if (reduce_by_key((unsigned long long)V.loss, l2)) atomicAdd(V.loss, l2[0]);
             }
         }
         const GradSink sink{V.grad, nullptr, 0u, nullptr};
