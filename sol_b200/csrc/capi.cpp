@@ -512,7 +512,7 @@ int sol_gpu_trace(SolGpuScene* scene, const SolGpuRay* rays_device, uint32_t cou
         cudaError_t e = cudaMemsetAsync(hits_device, 0xff, sizeof(SolGpuHit) * count, static_cast<cudaStream_t>(stream));
         return e == cudaSuccess ? SOL_GPU_OK : cuda_fail(e, "cudaMemsetAsync");
     }
-    cudaError_t e = launch_trace(scene->view, rays_device, count, any_hit != 0, hits_device,
+    cudaError_t e = launch_trace(scene->view, rays_device, count, any_hit != 0, hits_device, scene->num_sms,
                                  static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? SOL_GPU_OK : cuda_fail(e, "trace launch");
 }

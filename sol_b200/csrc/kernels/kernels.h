@@ -135,7 +135,7 @@ cudaError_t launch_sum_items_views(const WfView* views, uint32_t num_views, uint
 
 /// K9: closest-hit or any-hit queries for a batch of rays.
 cudaError_t launch_trace(const SceneView& s, const SolGpuRay* rays, uint32_t count, bool any_hit,
-                         SolGpuHit* hits, cudaStream_t stream);
+                         SolGpuHit* hits, int sms, cudaStream_t stream);
 
 /// Launches `kernel` with an L2 access-policy window (persisting hits on
 /// l2.base .. + l2.bytes, streaming misses) when l2.bytes > 0, otherwise plainly.
