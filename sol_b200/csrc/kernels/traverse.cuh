@@ -143,8 +143,17 @@ __device__ __forceinline__ F2 fma2(F2 x, float y, F2 z) {
     return r;
 }
 
-/// Reciprocal direction of the packed box test.  As safe_inverse with a floor
-/// of 1e-24: with centres and half sizes of at most kBoxRange (larger boxes are
+/// 1 / v within one unit in the last place (one instruction; the correctly
+/// rounded division is a short program).
+__device__ __forceinline__ float rcp_approx(float v) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+/// Reciprocal direction of the packed box test, which needs no exact one (its
+/// error is part of the bound at child_boxes; frame 44.3 -> 43.9 ms, textured
+/// 547 -> 540 us against divisions).  As safe_inverse with a floor of 1e-24: with centres and half sizes of at most kBoxRange (larger boxes are
 /// stored as boundless), (centre - org) / direction of a ray that starts within
 /// that range stays finite, so no inf - inf arises where the exact form has
 /// infinities of two signs.
@@ -153,7 +162,7 @@ __device__ __forceinline__ Vec3 box_inverse(Vec3 d) {
     const float x = fabs_(d.x) > eps ? d.x : copysign_(eps, d.x);
     const float y = fabs_(d.y) > eps ? d.y : copysign_(eps, d.y);
     const float z = fabs_(d.z) > eps ? d.z : copysign_(eps, d.z);
-    return vec3(1.0f / x, 1.0f / y, 1.0f / z);
+    return vec3(rcp_approx(x), rcp_approx(y), rcp_approx(z));
 }
 
 /// child_slabs on a DBoxNode: per axis both children's centre distances
@@ -166,11 +175,12 @@ __device__ __forceinline__ Vec3 box_inverse(Vec3 d) {
 /// of which the frame's share is 0.8 ms).
 ///
 /// Conservative: with eps = 2^-24, D = |c - o| / |d| and H = h / |d|, either
-/// distance errs by at most (3 D + H + |distance|) eps (subtraction, 1/d and
-/// multiplication on the first term, 1/d on the second, the sum's rounding).
-/// pack_boxes enlarges h by 16 eps, which covers D <= H; beyond, |distance| =
-/// D - H and half of the exit's widening (13 eps in all) covers the rest, since
-/// 16 + 6.5 (D / H - 1) >= 4 D / H + 2.
+/// distance errs by at most (4 D + 2 H + |distance|) eps (subtraction, 1/d within
+/// 2 eps and multiplication on the first term, 1/d on the second, the sum's
+/// rounding).  pack_boxes enlarges h by 16 eps, which covers D <= H; beyond,
+/// |distance| <= D + H and half of the exit's widening (13 eps in all) of a
+/// distance of at least D - H covers the rest, since 16 + 6.5 (D / H - 1) >=
+/// 5 D / H + 3.
 __device__ __forceinline__ void child_boxes(float4 x, float4 y, float4 z, Vec3 org, Vec3 idir, float tmin, float tmax,
                                             float& n0, float& f0, float& n1, float& f1) {
     const float ax = fabsf(idir.x), ay = fabsf(idir.y), az = fabsf(idir.z);

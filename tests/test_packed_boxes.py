@@ -27,6 +27,8 @@ def passes(lo, hi, o, d, tmin, tmax):
     c, h = pack(lo, hi)
     d = np.where(np.abs(d) > F(1e-24), d, np.copysign(F(1e-24), d)).astype(F)
     idir = (F(1.0) / d).astype(F)
+    ulp = np.random.default_rng(1).integers(-1, 2, d.shape)   # the reciprocal is within one unit in the last place
+    idir = np.where(ulp < 0, np.nextafter(idir, F(0)), np.where(ulp > 0, np.nextafter(idir, F(np.inf) * np.sign(idir)), idir))
     with np.errstate(over="ignore", invalid="ignore"):
         t = ((c - o).astype(F) * idir).astype(F)
         n = np.fmax(fma(h, -np.abs(idir), t).max(axis=1), tmin)
