@@ -386,7 +386,7 @@ wf_shade(const WfParams* __restrict__ Pp, const __grid_constant__ WfSceneTable s
         ps.path_len = __float_as_uint(c4.w);
         ps.rng.state = P.rng[slot];
         VertexOut vo;
-        shade_vertex<kBasic>(sv, P.cfg, 1.0f / (float)sv.num_lights, tri, h.y, ps, vo, true, h.z, h.w);
+        shade_vertex<kBasic ? kShadeBasic : kShadeFull>(sv, P.cfg, 1.0f / (float)sv.num_lights, tri, h.y, ps, vo, true, h.z, h.w);
         bool end = vo.end;
         if (!end) {
             ++ps.path_len;
