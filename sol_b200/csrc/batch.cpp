@@ -67,7 +67,7 @@ size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 size_t pool_bytes(uint32_t c) {
     size_t b = 0;
-    b += 9 * align256(sizeof(float4) * (size_t)c);                    // thru color ray_o[2] ray_d[2] sh_o sh_d sh_c
+    b += 9 * align256(sizeof(float4) * (size_t)c);                    // state (2) ray_o[2] ray_d[2] sh_o sh_d sh_c
     b += align256(sizeof(unsigned long long) * (size_t)c);            // rng
     b += align256(sizeof(uint2) * (size_t)c);                         // item
     b += align256(sizeof(float4) * (size_t)c);                        // hit
@@ -97,8 +97,7 @@ int alloc_pool(SolGpuBatch* b, uint32_t capacity) {
     auto take = [&](size_t bytes) { char* r = p; p += align256(bytes); return r; };
     const size_t c = capacity;
     WfParams& h = b->host;
-    h.thru = reinterpret_cast<float4*>(take(sizeof(float4) * c));
-    h.color = reinterpret_cast<float4*>(take(sizeof(float4) * c));
+    h.state = reinterpret_cast<float4*>(take(2 * sizeof(float4) * c));
     h.rng = reinterpret_cast<unsigned long long*>(take(sizeof(unsigned long long) * c));
     h.item = reinterpret_cast<uint2*>(take(sizeof(uint2) * c));
     for (int k = 0; k < 2; ++k) {

@@ -154,8 +154,8 @@ __device__ __forceinline__ uint32_t restart_slot(const WfParams& P, const WfView
         it = make_uint2(vi, local);
         col = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (P.cfg.max_path_len == 0) continue;   // empty path: black, written above
-        P.thru[slot] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
-        P.color[slot] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(0u));
+        P.state[2 * slot] = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+        P.state[2 * slot + 1] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(0u));
         P.rng[slot] = ps.rng.state;
         const uint32_t q = append(&ctr->extend[qp]);
         P.ray_o[qp][q] = make_float4(ps.org.x, ps.org.y, ps.org.z, ps.tmin);
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(256) wf_generate(const WfParams* __restrict__ 
         const uint32_t i = base + threadIdx.x;
         if (i >= n) continue;
         const uint32_t slot = P.q_ended[p][i];
-        paths += restart_slot(P, views, slot, P.color[slot], p);
+        paths += restart_slot(P, views, slot, P.state[2 * slot + 1], p);
     }
     paths = warp_sum(paths);
     if (lane_id() == 0 && paths) atomicAdd(&ctr->paths, paths);
@@ -368,7 +368,7 @@ wf_shade(const WfParams* __restrict__ Pp, const __grid_constant__ WfSceneTable s
         if (tri < 0) {   // path_tracer.cpp:43-44: no hit, the path ends
             if (packed) P.alt[1][i].w = -1.0f;   // no shadow ray at this extend position
 #if SOL_WF_SHADE_RESTART
-            paths += restart_slot(P, P.views, slot, P.color[slot], q);
+            paths += restart_slot(P, P.views, slot, P.state[2 * slot + 1], q);
 #else
             P.q_ended[q][append(&ctr->ended[q])] = slot;
 #endif
@@ -376,7 +376,7 @@ wf_shade(const WfParams* __restrict__ Pp, const __grid_constant__ WfSceneTable s
         }
         const SceneView& sv = scenes.v[tag >> kWfSlotBits];
         PathState ps;
-        const float4 t4 = P.thru[slot], c4 = P.color[slot];
+        const float4 t4 = P.state[2 * slot], c4 = P.state[2 * slot + 1];
         ps.org = vec3(o.x, o.y, o.z);
         ps.tmin = o.w;
         ps.dir = vec3(d.x, d.y, d.z);
@@ -392,9 +392,9 @@ wf_shade(const WfParams* __restrict__ Pp, const __grid_constant__ WfSceneTable s
             ++ps.path_len;
             end = ps.path_len >= P.cfg.max_path_len;
         }
-        P.color[slot] = make_float4(ps.color.r, ps.color.g, ps.color.b, __uint_as_float(ps.path_len));
+        P.state[2 * slot + 1] = make_float4(ps.color.r, ps.color.g, ps.color.b, __uint_as_float(ps.path_len));
         if (!end) {
-            P.thru[slot] = make_float4(ps.T.r, ps.T.g, ps.T.b, ps.pdf_prev);
+            P.state[2 * slot] = make_float4(ps.T.r, ps.T.g, ps.T.b, ps.pdf_prev);
             P.rng[slot] = ps.rng.state;
             const uint32_t j = append(&ctr->extend[q]);
             P.ray_o[q][j] = make_float4(ps.org.x, ps.org.y, ps.org.z, ps.tmin);
@@ -445,8 +445,8 @@ wf_shadow(const WfParams* __restrict__ Pp, const __grid_constant__ WfSceneTable 
     auto finish = [&](uint32_t i, const Traversal<true, false, true, false>& tr) {
         const uint32_t slot = __float_as_uint(P.sh_o[i].w) & kWfSlotMask;
         if (tr.hit < 0) {
-            const float4 c = P.color[slot], a = P.sh_c[i];
-            P.color[slot] = make_float4(c.x + a.x, c.y + a.y, c.z + a.z, c.w);
+            const float4 c = P.state[2 * slot + 1], a = P.sh_c[i];
+            P.state[2 * slot + 1] = make_float4(c.x + a.x, c.y + a.y, c.z + a.z, c.w);
         }
         if (P.sh_d[i].w != 0.0f) P.q_ended[q][append(&ctr->ended[q])] = slot;
     };

@@ -155,8 +155,10 @@ struct WfParams {
     const WfView* views;
     WfCounters* ctr;
     // per slot
-    float4* thru;            // throughput, pdf_prev
-    float4* color;           // radiance gathered so far, path_len (bits)
+    // Two vectors per slot, one 32-byte sector: throughput and pdf_prev; radiance
+    // gathered so far and path_len (bits).  Slots come in any order, so each
+    // separate 16-byte access would move a sector of its own, half unused.
+    float4* state;
     unsigned long long* rng;
     uint2* item;             // the slot's work item: view, item within the view (view = idle: none)
     // per queue position
