@@ -119,8 +119,11 @@ int configure_launch(SolGpuBatch* b) {
     int block = (int)(b->opts.block_size ? b->opts.block_size : 128);
     if (block != 64 && block != 128 && block != 256) return fail(SOL_GPU_ERR_INVALID_ARG, "block_size must be 64, 128 or 256");
     if (block == b->launch_block) return SOL_GPU_OK;
+    uint64_t bytes = 0;   // what the traversal stages read of the scenes
+    for (const SceneView& v : b->h_scenes) bytes += sizeof(DBoxNode) * (uint64_t)v.num_nodes + sizeof(DTri) * (uint64_t)v.num_tris;
+    b->launch.large = bytes > kWfCachedSceneBytes;
     for (int s = 0; s < 4; ++s) {
-        int per_sm = wavefront_blocks_per_sm(s, block);
+        int per_sm = wavefront_blocks_per_sm(s, block, b->launch.large);
         if (per_sm <= 0) return fail(SOL_GPU_ERR_CUDA, "wavefront occupancy query failed");
         b->launch.grid[s] = per_sm * b->num_sms;
         b->launch.block[s] = block;

@@ -305,7 +305,8 @@ __device__ __forceinline__ void trace_queue(const WfSceneTable& scenes, uint32_t
 
 /// K3: closest hit for every queued ray, written in queue order; hits binned by
 /// BSDF kind (K6) when the queue is long enough.
-__global__ void __launch_bounds__(256, kWfTraceMinBlocks)
+template <int kMinBlocks>
+__global__ void __launch_bounds__(256, kMinBlocks)
 wf_extend(const WfParams* __restrict__ Pp, const __grid_constant__ WfSceneTable scenes) {
     const WfParams& P = *Pp;
     WfCounters* ctr = P.ctr;
@@ -428,7 +429,8 @@ wf_shade(const WfParams* __restrict__ Pp, const __grid_constant__ WfSceneTable s
 }
 
 /// K4: shadow rays; the light sample's contribution is added when unoccluded.
-__global__ void __launch_bounds__(256, kWfTraceMinBlocks)
+template <int kMinBlocks>
+__global__ void __launch_bounds__(256, kMinBlocks)
 wf_shadow(const WfParams* __restrict__ Pp, const __grid_constant__ WfSceneTable scenes) {
     const WfParams& P = *Pp;
     WfCounters* ctr = P.ctr;
@@ -628,6 +630,11 @@ __global__ void wf_advance(const WfParams* __restrict__ Pp, cudaGraphConditional
     if (use_handle) cudaGraphSetConditional(handle, more ? 1u : 0u);
 }
 
+/// The traversal stages' builds (see kWfTraceMinBlocks).
+using WfStageFn = void (*)(const WfParams*, const WfSceneTable);
+WfStageFn extend_fn(bool large) { return large ? wf_extend<kWfTraceLargeMinBlocks> : wf_extend<kWfTraceMinBlocks>; }
+WfStageFn shadow_fn(bool large) { return large ? wf_shadow<kWfTraceLargeMinBlocks> : wf_shadow<kWfTraceMinBlocks>; }
+
 /// Dynamic shared memory of a traversal-stage block of `block` threads.
 size_t trace_smem(int block) { return kWfSharedStack ? sizeof(int) * kSharedStackDepth * (size_t)block : 0; }
 
@@ -637,22 +644,25 @@ size_t trace_smem(int block) { return kWfSharedStack ? sizeof(int) * kSharedStac
 cudaError_t allow_trace_smem() {
     const int bytes = (int)trace_smem(256);
     if (bytes <= 48 * 1024) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(wf_extend, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(wf_shadow, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaError_t e = cudaSuccess;
+    for (bool large : {false, true}) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(extend_fn(large), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(shadow_fn(large), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    }
     return e;
 }
 
 }  // namespace
 
-int wavefront_blocks_per_sm(int stage, int block) {
+int wavefront_blocks_per_sm(int stage, int block, bool large) {
     int n = 0;
     if (allow_trace_smem() != cudaSuccess) return -1;
     cudaError_t e = cudaSuccess;
     switch (stage) {
         case 0: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wf_generate, block, 0); break;
-        case 1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wf_extend, block, trace_smem(block)); break;
+        case 1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, extend_fn(large), block, trace_smem(block)); break;
         case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wf_shade<false>, block, 0); break;
-        default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, wf_shadow, block, trace_smem(block)); break;
+        default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, shadow_fn(large), block, trace_smem(block)); break;
     }
     return e == cudaSuccess ? n : -1;
 }
@@ -694,12 +704,12 @@ cudaError_t launch_wf_iteration(WfParams* params, const WfSceneTable& scenes, bo
     const int sms = L.sms > 0 ? L.sms : 1;
     wf_generate<<<L.grid[0], L.block[0], 0, stream>>>(params);
     if (ray_sort) launch_sort(params, 0, sms, stream);
-    wf_extend<<<L.grid[1], L.block[1], trace_smem(L.block[1]), stream>>>(params, scenes);
+    extend_fn(L.large)<<<L.grid[1], L.block[1], trace_smem(L.block[1]), stream>>>(params, scenes);
     if (basic) wf_shade<true><<<L.grid[2], L.block[2], 0, stream>>>(params, scenes);
     else wf_shade<false><<<L.grid[2], L.block[2], 0, stream>>>(params, scenes);
     if (packed_shadows) wf_shadow_compact<<<4 * sms, 1024, 0, stream>>>(params);
     if (ray_sort) launch_sort(params, 1, sms, stream);
-    wf_shadow<<<L.grid[3], L.block[3], trace_smem(L.block[3]), stream>>>(params, scenes);
+    shadow_fn(L.large)<<<L.grid[3], L.block[3], trace_smem(L.block[3]), stream>>>(params, scenes);
     wf_advance<<<1, 1, 0, stream>>>(params, handle, use_handle);
     return cudaGetLastError();
 }

@@ -27,9 +27,14 @@ constexpr int kWfRefillBelow = SOL_WF_REFILL_BELOW;
 /// 3 (up to 80 registers, nothing spilled): the stages are chains of dependent
 /// node fetches that spilling (6 blocks, 40 registers) lengthens, and every
 /// bounce launches the full grid, so fewer blocks also cost less where the
-/// queues are short.  24 views (about 25M paths) 9.86 ms at 6 blocks, 8.91 at
-/// 4, 8.73 at 3, 8.82 at 2; 4 small views 1.25, 1.06, 0.94 ms.
+/// queues are short.  24 views (19M paths) of 262k triangles 8.89 ms at 6
+/// blocks, 8.65 at 5, 8.56 at 4, 8.52 at 3.  Scenes that L2 does not hold beside
+/// the queues (kWfCachedSceneBytes of nodes and triangles) wait for memory
+/// instead, which more warps hide: the same views of 1M triangles 12.43, 12.24,
+/// 12.58 and 12.98 ms, of 4.2M 25.28, 25.32, 26.64 and 28.71 ms.
 constexpr int kWfTraceMinBlocks = SOL_WF_TRACE_MIN_BLOCKS;
+constexpr int kWfTraceLargeMinBlocks = 5;
+constexpr uint64_t kWfCachedSceneBytes = 48ull << 20;
 
 #ifndef SOL_WF_SHADE_MIN_BLOCKS
 #define SOL_WF_SHADE_MIN_BLOCKS 2
@@ -177,9 +182,10 @@ struct WfLaunch {
     int grid[4];
     int block[4];
     int sms;                 // multiprocessors of the device (grids of the reordering kernels)
+    bool large;              // traversal stages at kWfTraceLargeMinBlocks
 };
 
-int wavefront_blocks_per_sm(int stage, int block);
+int wavefront_blocks_per_sm(int stage, int block, bool large);
 cudaError_t launch_wf_init(const WfParams* params, uint32_t capacity, cudaStream_t stream);
 /// One bounce of the wavefront: generate, extend, shade, shadow, advance.
 /// `basic`: every scene has basic shading (shade's build without image

@@ -25,3 +25,21 @@ def test_films_match_plain_renders(built, sizes, host_loop):
         pt.render_device(want.data_ptr(), w, h, 2, spp)
         torch.cuda.synchronize()
         assert np.array_equal(f.cpu().numpy(), want.cpu().numpy())
+
+
+def test_large_scene_build_matches_plain_render(built):
+    """Nodes and triangles beyond 48 MB: the traversal stages' other build."""
+    import torch
+    from sol_b200 import capi, scenes
+    from sol_b200.renderer import BatchRenderer, GpuPathTracer, GpuScene
+    gs = GpuScene(scenes.sphere_field(28, seed=3), gpu_bvh=True)
+    info = gs.info()
+    assert 64 * info.num_nodes + 48 * info.num_triangles > 48 << 20
+    w, h, spp = 93, 61, 3
+    film, want = torch.zeros((3, h, w), device="cuda"), torch.zeros((3, h, w), device="cuda")
+    b = BatchRenderer([gs], schedule=capi.BATCH_WAVEFRONT)
+    b.render(scenes.SPHERES_CONFIG, b.views([(0, gs.scene.camera, w, h, 0, spp, film.data_ptr())]))
+    b.stats()
+    GpuPathTracer(gs, scenes.SPHERES_CONFIG).render_device(want.data_ptr(), w, h, 0, spp)
+    torch.cuda.synchronize()
+    assert want.any() and torch.equal(film, want)
