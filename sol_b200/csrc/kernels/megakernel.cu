@@ -9,8 +9,8 @@
 // exhausted.  One lane owns a pixel for all of its samples, which keeps the
 // per-pixel sum in SoL's sample order and the result bit-identical to the host.
 //
-// Renders of more than one sample use the split schedule instead (the host's
-// AUTO choice): a work item is one (pixel, sample), so the samples of a pixel
+// Single samples take the lean kernel below.  Renders of more than one sample
+// use the split schedule (the host's AUTO choice), also on the lean kernel: a work item is one (pixel, sample), so the samples of a pixel
 // run on different lanes; each writes its path's colour (0 + colour, as the
 // per-pixel sum starts) to a scratch plane of its sample, and sum_samples adds
 // each pixel's colours in sample order, which is the same sequence of
