@@ -574,6 +574,12 @@ int sol_gpu_adjoint(SolGpuScene* scene, const SolGpuCamera* camera, const SolGpu
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     cudaError_t e = cudaMemsetAsync(scene->counters, 0, sizeof(DeviceCounters), st);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync");
+    if (sample_count == 0) {   // no paths, nothing to add (and no chunk of samples to divide by)
+        cudaEventRecord(scene->ev_start, st);
+        cudaEventRecord(scene->ev_stop, st);
+        scene->rendered = true;
+        return SOL_GPU_OK;
+    }
     const uint32_t n_shared = (uint32_t)std::min<uint64_t>(scene->constants_count, kAdjointMaxSharedParams);
     const AdjointBuild build = adjoint_build((uint64_t)width * height * sample_count, config->max_path_len, scene->num_sms);
     const int per_sm = adjoint_blocks_per_sm(build, n_shared);

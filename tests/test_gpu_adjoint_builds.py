@@ -61,3 +61,14 @@ def test_fused_matches_render_loss_and_adjoint(built, w, h, spp):
     a, b = loss.tolist()
     assert abs(a - b) <= 1e-6 * abs(b)   # the residual's rounding (sum * (1 / spp) in either order)
     assert _close(g.double().cpu().numpy(), g2.double().cpu().numpy())
+
+
+def test_no_samples_add_nothing(built):
+    import torch
+    pt = _tracer()
+    grad = torch.full((pt.scene.param_layout()[0],), 0.5, device="cuda")
+    dl = torch.ones((3, 9, 7), device="cuda")
+    pt.adjoint(dl.data_ptr(), grad.data_ptr(), 7, 9, 2, 0)
+    st = pt.stats()
+    assert (st.paths, st.rays) == (0, 0)
+    assert (grad == 0.5).all()
