@@ -444,10 +444,15 @@ __device__ void restructure(const Tree& t, int root, float root_cost, Treelet& w
 /// is a leaf; then the warp restructures, one after another, the treelets that
 /// its lanes' nodes root, and every lane goes on to its node's parent.  A walk
 /// longer than any tree of n leaves sets `*fail` (the build is then rejected).
-/// All lanes stay in the loop until the warp's last walk ends.  Nodes are
-/// published by the fence and the atomic of the next arrival; a treelet's
-/// writes come from several lanes, each fencing its own before the warp
-/// barrier.
+/// All lanes stay in the loop until the warp's last walk ends.
+///
+/// Memory order: a node is published by the fence and the atomic of the next
+/// arrival.  The lane that arrives second fences after its atomic, which orders
+/// its own reads; the other lanes of the warp, which read the treelet's nodes
+/// and boxes (other blocks' writes) too, are ordered after that fence, and
+/// after its stores of the node, by the warp barrier before the vote (a vote or
+/// a shuffle orders no memory).  A treelet's writes come from several lanes,
+/// each fencing its own before the warp barrier that ends it.
 __global__ void __launch_bounds__(kBottomUpBlock)
 bottom_up(Tree t, int n, unsigned int* __restrict__ arrived, unsigned int* __restrict__ fail) {
     __shared__ Treelet treelets[kBottomUpBlock / 32];
@@ -487,6 +492,7 @@ bottom_up(Tree t, int n, unsigned int* __restrict__ arrived, unsigned int* __res
                 t.cost[node] = cost;
                 t.leaf[node] = leaf ? 1 : 0;
             }
+            __syncwarp();
             unsigned todo = __ballot_sync(all, node >= 0 && count >= kTreeletMinCount);
             while (todo) {
                 const int src = __ffs(todo) - 1;
