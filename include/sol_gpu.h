@@ -506,7 +506,8 @@ int sol_gpu_batch_forward_adjoint(SolGpuBatch* batch, const SolGpuConfig* config
  * counters in the array are cleared by the call itself.  Calls share the
  * array, so calls that can overlap on the GPU (different streams without
  * ordering, different host threads) race: order them.  The first call on a
- * device looks up the array's address; make it before any stream capture.
+ * device looks up the array's address and makes the kernels of every call size
+ * resident; make it (zero views will do) before any stream capture.
  * The tables reach the array as kernel parameters of a small copy kernel (no
  * copy from pageable host memory).  With lazy module loading (the CUDA 12
  * default) the library's device image and the array become resident on a

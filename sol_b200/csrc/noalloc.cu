@@ -20,8 +20,9 @@
 // reuses the same array, so two calls that can overlap on the GPU (on two
 // streams with no ordering between them, or from two host threads) race on
 // it; the caller must order them.  The first call on a device looks the
-// array's device address up (cudaGetSymbolAddress); make that first call
-// before any stream capture.
+// array's device address up (cudaGetSymbolAddress) and runs every kernel that
+// later calls may launch once without work, whatever its own size; make that
+// first call (zero views will do) before any stream capture.
 //
 // The tables are built on the host and reach the array as kernel parameters:
 // a small copy kernel takes up to 30 KiB of them by value per launch and
@@ -99,17 +100,34 @@ constexpr int kMaxDevices = 64;
 std::mutex g_setup_mutex;
 unsigned char* g_scratch_ptr[kMaxDevices] = {};
 
-/// Device address of the scratch array on the current device, looked up once
-/// per device (the first call on a device does this; make that first call before
-/// any stream capture).
-int scratch_address(int device, unsigned char** out) {
+/// Device address of the scratch array on the current device.  The first call on
+/// a device (make it before any stream capture) also makes everything resident
+/// that later calls of any size launch: it runs the copy kernel and both builds
+/// of the fused kernel once, with no work items, on `stream`.  A build that
+/// first ran in a later call would be loaded there, and its local memory, when
+/// larger than what the context holds, allocated there.
+int scratch_address(int device, cudaStream_t stream, unsigned char** out) {
     if (device < 0 || device >= kMaxDevices) return fail(SOL_GPU_ERR_UNSUPPORTED, "device ordinal out of range");
     std::lock_guard<std::mutex> lock(g_setup_mutex);
     if (!g_scratch_ptr[device]) {
         void* p = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
         if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(scratch)");
-        g_scratch_ptr[device] = static_cast<unsigned char*>(p);
+        unsigned char* scratch = static_cast<unsigned char*>(p);
+        int num_sms = 0;
+        e = cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, device);
+        alignas(16) const unsigned char zero[align256_(sizeof(DeviceCounters))] = {};
+        if (e == cudaSuccess) e = upload(zero, kCountersOffset, sizeof(DeviceCounters), scratch, stream);
+        for (AdjointBuild build : {AdjointBuild::kSmall, AdjointBuild::kFull}) {
+            const int per_sm = e == cudaSuccess ? fused_blocks_per_sm(build) : 0;
+            if (e == cudaSuccess && per_sm <= 0) return fail(SOL_GPU_ERR_CUDA, "fused kernel occupancy query failed");
+            if (e == cudaSuccess)
+                e = launch_fused_forward_adjoint(nullptr, 0, 0, nullptr, DConfig{},
+                                                 reinterpret_cast<DeviceCounters*>(scratch + kCountersOffset), build,
+                                                 per_sm * num_sms, stream);
+        }
+        if (e != cudaSuccess) return cuda_fail(e, "first launch of the fused kernels");
+        g_scratch_ptr[device] = scratch;
     }
     *out = g_scratch_ptr[device];
     return SOL_GPU_OK;
@@ -171,11 +189,11 @@ extern "C" int sol_gpu_batch_forward_adjoint_noalloc(SolGpuScene* const* scenes,
     }
     DeviceGuard guard(device);
     if (guard.err != cudaSuccess) return cuda_fail(guard.err, "cudaSetDevice");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
     unsigned char* scratch = nullptr;
-    int rc = scratch_address(device, &scratch);
+    int rc = scratch_address(device, st, &scratch);
     if (rc != SOL_GPU_OK) return rc;
     if (num_views == 0) return SOL_GPU_OK;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
     SceneView* d_scenes = reinterpret_cast<SceneView*>(scratch + kScenesOffset);
     AdjView* d_views = reinterpret_cast<AdjView*>(scratch + kViewsOffset);
     DeviceCounters* d_ctr = reinterpret_cast<DeviceCounters*>(scratch + kCountersOffset);
