@@ -498,6 +498,19 @@ SOL_HD Vec3 safe_inverse(Vec3 d) {
     return vec3(1.0f / x, 1.0f / y, 1.0f / z);
 }
 
+/// Whether boxes stored as centre and half size (DBoxNode) may be tested along
+/// direction d.  The range keeps every quotient of a distance of at most 2e13 (the
+/// largest stored box) and a component finite, and those of scenes down to 1e-15
+/// out of the subnormal numbers.  A component below 2^-32 of the largest (zero
+/// above all) leaves the ray in a face of a box all along where its origin lies in
+/// it, and whether that is inside is decided by the last bit of the face, which
+/// a centre and a half size do not hold.
+SOL_HD bool boxes_take(Vec3 d) {
+    const float x = fabs_(d.x), y = fabs_(d.y), z = fabs_(d.z);
+    const float least = fminf(fminf(x, y), z), most = fmaxf(fmaxf(x, y), z);
+    return least >= 0x1p-32f * most && most >= 0x1p-47f && most <= 0x1p50f;
+}
+
 /// Widening factor applied to the exit distance of every slab test so that
 /// rounding in the box test never culls a box that the exact ray touches
 /// (Ize: "Robust BVH Ray Traversal", JCGT 2(2), 2013: 1 + 2 gamma(3)).

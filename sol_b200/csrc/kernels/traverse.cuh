@@ -17,8 +17,9 @@
 //          in an order that may differ from the host's where two boxes begin at
 //          (nearly) equal distances.  The closest hit is the same unless several
 //          triangles are hit at exactly the closest distance; a ray that meets
-//          that case is traced again in the exact form (closest_exact).  A shadow
-//          ray only asks whether anything is hit, which no order changes.
+//          that case is traced again in the exact form (closest_exact), and so is
+//          one whose direction the packed test does not take (boxes_take).  A
+//          shadow ray only asks whether anything is hit, which no order changes.
 #pragma once
 
 #include "../core/layout.h"
@@ -153,17 +154,8 @@ __device__ __forceinline__ float rcp_approx(float v) {
 
 /// Reciprocal direction of the packed box test, which needs no exact one (its
 /// error is part of the bound at child_boxes; frame 44.3 -> 43.9 ms, textured
-/// 547 -> 540 us against divisions).  As safe_inverse with a floor of 1e-24: with centres and half sizes of at most kBoxRange (larger boxes are
-/// stored as boundless), (centre - org) / direction of a ray that starts within
-/// that range stays finite, so no inf - inf arises where the exact form has
-/// infinities of two signs.
-__device__ __forceinline__ Vec3 box_inverse(Vec3 d) {
-    const float eps = 1e-24f;
-    const float x = fabs_(d.x) > eps ? d.x : copysign_(eps, d.x);
-    const float y = fabs_(d.y) > eps ? d.y : copysign_(eps, d.y);
-    const float z = fabs_(d.z) > eps ? d.z : copysign_(eps, d.z);
-    return vec3(rcp_approx(x), rcp_approx(y), rcp_approx(z));
-}
+/// 547 -> 540 us against divisions).  For directions that boxes_take.
+__device__ __forceinline__ Vec3 box_inverse(Vec3 d) { return vec3(rcp_approx(d.x), rcp_approx(d.y), rcp_approx(d.z)); }
 
 /// child_slabs on a DBoxNode: per axis both children's centre distances
 /// (c - o) / d in one packed subtract and multiply, then entry and exit as
@@ -203,15 +195,16 @@ __device__ __forceinline__ void load_boxes(const DBoxNode* n, float4& x, float4&
         : "=f"(z.x), "=f"(z.y), "=f"(z.z), "=f"(z.w), "=r"(ref.x), "=r"(ref.y) : "l"(n));
 }
 
-/// Set in Traversal::hit when another triangle was hit at exactly the distance
-/// of the closest one (positions in leaf order stay below 2^28).
-constexpr int kTieBit = 1 << 30;
+/// Set in Traversal::hit when the exact traversal has to find the hit: another
+/// triangle was hit at exactly the distance of the closest one (positions in
+/// leaf order stay below 2^28), or the direction is none that boxes_take.
+constexpr int kRedoBit = 1 << 30;
 
 /// BVH traversal of one ray as a resumable state: start() sets it up, run()
 /// advances it.  For kAnyHit the first triangle hit inside (tmin, tmax) is
 /// kept; otherwise the closest one, with `tmax` shrunk to its distance.  `hit`
-/// is the triangle's position in leaf order, or -1.  A packed closest-hit
-/// traversal (kExact = false) must be followed by resolve().
+/// is the triangle's position in leaf order, or -1.  A packed traversal
+/// (kExact = false) must be followed by resolve().
 ///
 /// A packed any-hit traversal takes the first child first, whichever is nearer:
 /// the answer does not depend on the order, and not ordering the children saves
@@ -251,6 +244,10 @@ struct Traversal {
         steps = 0;
         node = active ? 0 : kStackSentinel;
         stack.put(sp++, kStackSentinel);
+        if (!kExact && active && !boxes_take(d)) {   // nothing to run, resolve() traces the ray
+            node = kStackSentinel;
+            hit = kRedoBit;
+        }
     }
 
     __device__ __forceinline__ bool fail(unsigned int* fault, unsigned int bit) {
@@ -332,10 +329,10 @@ struct Traversal {
                         tmax = t;
                         hu = u;
                         hv = w;
-                    } else if (hit >= 0 && (hit & ~kTieBit) != (int)i) {
+                    } else if (hit >= 0 && (hit & ~kRedoBit) != (int)i) {
                         // (Without a hit, tmax is the ray's own end, which is no hit; a tree of
                         // one leaf has it as both children of its root.)
-                        hit |= kTieBit;
+                        hit |= kRedoBit;
                     }
                 }
             }
@@ -347,14 +344,14 @@ struct Traversal {
         return true;
     }
 
-    /// After a packed closest-hit traversal that began with the end `t1`: when
-    /// several triangles are hit at the closest distance, the one that the
-    /// exact traversal finds.
+    /// After a packed traversal that began with the end `t1`: where kRedoBit is
+    /// set, the hit that the exact traversal finds.
     __device__ __forceinline__ void resolve(const SceneView& s, float t1);
 };
 
-/// The closest hit of one ray by the exact traversal, out of line: only rays
-/// with several hits at exactly the closest distance come here.
+/// The closest hit of one ray by the exact traversal, out of line: only the few
+/// rays with kRedoBit come here.  (Whether there is any hit is the same question
+/// for both queries: they part only after the first.)
 struct ExactHit { int hit; float t, u, v; };
 static __device__ __noinline__ ExactHit closest_exact(const DNode* nodes, const DTri* tris, uint32_t num_nodes,
                                                       uint32_t num_tris, uint32_t max_steps, unsigned int* fault,
@@ -369,7 +366,7 @@ static __device__ __noinline__ ExactHit closest_exact(const DNode* nodes, const 
 
 template <bool kAnyHit, bool kCount, bool kYield, bool kExact>
 __device__ __forceinline__ void Traversal<kAnyHit, kCount, kYield, kExact>::resolve(const SceneView& s, float t1) {
-    if (kAnyHit || kExact || hit < kTieBit) return;
+    if (kExact || hit < kRedoBit) return;
     const ExactHit e = closest_exact(s.nodes(), s.tris, s.num_nodes, s.num_tris, s.max_steps, s.fault, org, dir, tmin, t1);
     hit = e.hit;
     tmax = e.t;
