@@ -144,19 +144,6 @@ __device__ __forceinline__ F2 fma2(F2 x, float y, F2 z) {
     return r;
 }
 
-/// 1 / v within one unit in the last place (one instruction; the correctly
-/// rounded division is a short program).
-__device__ __forceinline__ float rcp_approx(float v) {
-    float r;
-    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
-    return r;
-}
-
-/// Reciprocal direction of the packed box test, which needs no exact one (its
-/// error is part of the bound at child_boxes; frame 44.3 -> 43.9 ms, textured
-/// 547 -> 540 us against divisions).  For directions that boxes_take.
-__device__ __forceinline__ Vec3 box_inverse(Vec3 d) { return vec3(rcp_approx(d.x), rcp_approx(d.y), rcp_approx(d.z)); }
-
 /// child_slabs on a DBoxNode: per axis both children's centre distances
 /// (c - o) / d in one packed subtract and multiply, then entry and exit as
 /// that distance -+ h |1/d| in two packed fused multiply-adds: 12 packed
@@ -167,12 +154,14 @@ __device__ __forceinline__ Vec3 box_inverse(Vec3 d) { return vec3(rcp_approx(d.x
 /// of which the frame's share is 0.8 ms).
 ///
 /// Conservative: with eps = 2^-24, D = |c - o| / |d| and H = h / |d|, either
-/// distance errs by at most (4 D + 2 H + |distance|) eps (subtraction, 1/d within
-/// 2 eps and multiplication on the first term, 1/d on the second, the sum's
-/// rounding).  pack_boxes enlarges h by 16 eps, which covers D <= H; beyond,
-/// |distance| <= D + H and half of the exit's widening (13 eps in all) of a
-/// distance of at least D - H covers the rest, since 16 + 6.5 (D / H - 1) >=
-/// 5 D / H + 3.
+/// distance errs by at most (3 D + H + |distance|) eps (subtraction, 1/d and
+/// multiplication on the first term, 1/d on the second, the sum's rounding).
+/// pack_boxes enlarges h by 16 eps, which covers D <= H; beyond, |distance| <=
+/// D + H and half of the exit's widening (13 eps in all) of a distance of at
+/// least D - H covers the rest, since 16 + 6.5 (D / H - 1) >= 4 D / H + 2, with
+/// at least 2.5 D eps to spare for the triangle test's own rounding.  (The
+/// approximate reciprocal errs by 2 eps, which takes 1 D of that; it gained 1 %
+/// on the frame.)
 __device__ __forceinline__ void child_boxes(float4 x, float4 y, float4 z, Vec3 org, Vec3 idir, float tmin, float tmax,
                                             float& n0, float& f0, float& n1, float& f1) {
     const float ax = fabsf(idir.x), ay = fabsf(idir.y), az = fabsf(idir.z);
@@ -236,7 +225,7 @@ struct Traversal {
         dir = d;
         tmin = t0;
         tmax = t1;
-        idir = kExact ? safe_inverse(d) : box_inverse(d);
+        idir = kExact ? safe_inverse(d) : vec3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);   // the same where boxes_take(d)
         rs = make_shear(o, d);
         sp = 0;
         hit = -1;
