@@ -177,7 +177,7 @@ typedef struct SolGpuSceneInfo {
     uint32_t num_nodes;       /* inner nodes of the device BVH */
     uint32_t bvh_depth;
     float sah_cost;
-    uint64_t device_bytes;    /* node (both forms) + triangle + shading arrays */
+    uint64_t device_bytes;    /* node + triangle + shading arrays */
     float build_ms;           /* host BVH build + flatten */
 } SolGpuSceneInfo;
 

@@ -120,7 +120,7 @@ int configure_launch(SolGpuBatch* b) {
     if (block != 64 && block != 128 && block != 256) return fail(SOL_GPU_ERR_INVALID_ARG, "block_size must be 64, 128 or 256");
     if (block == b->launch_block) return SOL_GPU_OK;
     uint64_t bytes = 0;   // what the traversal stages read of the scenes
-    for (const SceneView& v : b->h_scenes) bytes += sizeof(DBoxNode) * (uint64_t)v.num_nodes + sizeof(DTri) * (uint64_t)v.num_tris;
+    for (const SceneView& v : b->h_scenes) bytes += sizeof(DNode) * (uint64_t)v.num_nodes + sizeof(DTri) * (uint64_t)v.num_tris;
     b->launch.large = bytes > kWfCachedSceneBytes;
     for (int s = 0; s < 4; ++s) {
         int per_sm = wavefront_blocks_per_sm(s, block, b->launch.large);

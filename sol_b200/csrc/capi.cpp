@@ -83,7 +83,7 @@ cudaError_t upload(T** dst, const std::vector<T>& src) {
 void release(SolGpuScene* s) {
     if (!s) return;
     DeviceGuard g(s->device);
-    cudaFree(s->boxes); cudaFree(s->tris); cudaFree(s->shade); cudaFree(s->tables); cudaFree(s->texels);
+    cudaFree(s->nodes); cudaFree(s->tris); cudaFree(s->shade); cudaFree(s->tables); cudaFree(s->texels);
     cudaFree(s->film_tmp); cudaFree(s->split_scratch); cudaFree(s->adj_texels4);
     if (s->film_host) cudaFreeHost(s->film_host);
     if (s->ev_start) cudaEventDestroy(s->ev_start);
@@ -242,7 +242,6 @@ int sol_gpu_scene_create_ex(const SolGpuSceneDesc* desc, int device, uint32_t fl
         cudaEventDestroy(b1);
         cudaFree(mesh);
         if (e == cudaSuccess) {
-            s->boxes = r.boxes;
             s->nodes = r.nodes;
             s->tris = r.tris;
             s->shade = r.shade;
@@ -258,15 +257,7 @@ int sol_gpu_scene_create_ex(const SolGpuSceneDesc* desc, int device, uint32_t fl
         }
     }
     if (!gpu_bvh) {
-        const size_t n = flat.nodes.size();
-        if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&s->boxes), n * (sizeof(DBoxNode) + sizeof(DNode)));
-        if (e == cudaSuccess) {
-            s->nodes = reinterpret_cast<DNode*>(s->boxes + n);
-            e = cudaMemcpy(s->nodes, flat.nodes.data(), n * sizeof(DNode), cudaMemcpyHostToDevice);
-        }
-        // On the stream of the copy: a copy from pageable memory may return before its
-        // data has reached the device, and other streams do not wait for it.
-        if (e == cudaSuccess) e = launch_pack_boxes(s->nodes, (uint32_t)n, s->boxes, cudaStreamLegacy);
+        if (e == cudaSuccess) e = upload(&s->nodes, flat.nodes);
         if (e == cudaSuccess) e = upload(&s->tris, flat.tris);
         if (e == cudaSuccess) e = upload(&s->shade, flat.shade);
     }
@@ -315,11 +306,12 @@ int sol_gpu_scene_create_ex(const SolGpuSceneDesc* desc, int device, uint32_t fl
             s->fault = reinterpret_cast<unsigned int*>(s->tables + fault);
         }
     }
-    // The uploads (and the box nodes made from them) are on the legacy stream, renders on any.
+    // A copy from pageable memory may return before its data has reached the device,
+    // and the streams that renders run on do not wait for it.
     if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (e != cudaSuccess) { int rc = cuda_fail(e, "scene upload"); release(s); return rc; }
 
-    s->view.boxes = s->boxes;
+    s->view.nodes = s->nodes;
     s->view.tris = s->tris;
     s->view.shade = s->shade;
     s->view.bsdfs = s->bsdfs;
@@ -344,7 +336,7 @@ int sol_gpu_scene_create_ex(const SolGpuSceneDesc* desc, int device, uint32_t fl
     s->info.num_nodes = (uint32_t)num_nodes;
     s->info.bvh_depth = flat.depth;
     s->info.sah_cost = flat.sah_cost;
-    s->info.device_bytes = num_nodes * (sizeof(DBoxNode) + sizeof(DNode)) + num_tris * (sizeof(DTri) + sizeof(DTriShade));
+    s->info.device_bytes = num_nodes * sizeof(DNode) + num_tris * (sizeof(DTri) + sizeof(DTriShade));
     s->info.build_ms = (float)flat.build_ms + gpu_build_ms;
 #if SOL_L2_PERSIST
     // Keep the upper BVH levels (stored first) in L2: raise this process's
@@ -361,7 +353,7 @@ int sol_gpu_scene_create_ex(const SolGpuSceneDesc* desc, int device, uint32_t fl
             cudaDeviceGetLimit(&have, cudaLimitPersistingL2CacheSize);
             const size_t bytes = (size_t)flat.top_nodes * sizeof(DNode);
             if (have > 0 && bytes > 0) {
-                s->l2.base = s->boxes;
+                s->l2.base = s->nodes;
                 s->l2.bytes = bytes;
                 s->l2.hit_ratio = (float)std::min(1.0, (double)have / (double)bytes);
             }

@@ -1,12 +1,7 @@
 // Device layout of an uploaded scene (shared by the host flattener and kernels).
 //
-//  boxes   : BVH2, one 64-byte record per inner node holding both child boxes
-//            as centre and half size and the child references, read as two
-//            32-byte vectors; what the renderers traverse.
-//  nodes   : the same hierarchy (same indices) with the boxes as lower and upper
-//            bounds, right behind `boxes`; what decides between hits at exactly
-//            equal distances, and what ray queries whose first hit is returned
-//            and the counting kernels traverse.
+//  nodes   : BVH2, one 64-byte record per inner node holding the boxes of both
+//            children and their references, read as two 32-byte vectors.
 //  tris    : one 48-byte record per triangle in BVH leaf order, the three
 //            vertices for the watertight test; the w lanes carry the caller's
 //            triangle index, the BSDF and the light of the triangle.
@@ -29,23 +24,13 @@ constexpr int32_t kStackSentinel = (int32_t)0x80000000;   // never a valid refer
 constexpr uint32_t kMaxTriangles = (1u << 28) - 2;
 constexpr int kTraversalStack = 64;                        // >= BVH depth - 1
 
-struct alignas(16) DNode {
+struct alignas(32) DNode {
     float b0[4];    // c0.lo.x, c0.hi.x, c0.lo.y, c0.hi.y
     float b1[4];    // c1.lo.x, c1.hi.x, c1.lo.y, c1.hi.y
     float b2[4];    // c0.lo.z, c0.hi.z, c1.lo.z, c1.hi.z
     int32_t ref[4]; // c0, c1, (unused), (unused)
 };
 static_assert(sizeof(DNode) == 64, "node layout");
-
-/// The children's boxes of a DNode as centre and half size (launch_pack_boxes),
-/// axis by axis so that both children sit in one register pair.
-struct alignas(32) DBoxNode {
-    float x[4];     // c0 centre, c1 centre, c0 half size, c1 half size
-    float y[4];
-    float z[4];
-    int32_t ref[4]; // as DNode::ref
-};
-static_assert(sizeof(DBoxNode) == 64, "box node layout");
 
 struct alignas(16) DTri {
     float v0[3]; uint32_t prim;   // caller's triangle index
@@ -113,7 +98,7 @@ struct DConfig {
 };
 
 struct SceneView {
-    const DBoxNode* boxes;   // num_nodes box nodes, then the num_nodes DNodes they were made from
+    const DNode* nodes;
     const DTri* tris;
     const DTriShade* shade;
     const DBsdf* bsdfs;
@@ -127,11 +112,6 @@ struct SceneView {
     uint32_t num_nodes;
     uint32_t max_steps;      // bound on traversal loop iterations (a tree never needs more)
     unsigned int* fault;     // device word; kernels OR kFault* bits into it instead of looping or reading out of bounds
-
-#if defined(__CUDACC__)
-    __host__ __device__
-#endif
-    const DNode* nodes() const { return reinterpret_cast<const DNode*>(boxes + num_nodes); }
 };
 
 /// Bits a kernel records in SceneView::fault when a self-check fails.

@@ -445,11 +445,11 @@ SOL_HD void edge_functions(const RayShear& r, Vec3 a, Vec3 b, Vec3 c,
 }
 
 /// Watertight intersection of a ray with triangle (v0, v1, v2), both sides.
-/// On a hit with tmin < t <= tmax returns true with the distance `t`
+/// On a hit strictly inside (tmin, tmax) returns true with the distance `t`
 /// (in units of the ray direction) and barycentrics u (weight of v1) and v
 /// (weight of v2).
-SOL_HD bool intersect_triangle_upto(const RayShear& r, Vec3 v0, Vec3 v1, Vec3 v2,
-                                    float tmin, float tmax, float* t_out, float* u_out, float* v_out) {
+SOL_HD bool intersect_triangle(const RayShear& r, Vec3 v0, Vec3 v1, Vec3 v2,
+                               float tmin, float tmax, float* t_out, float* u_out, float* v_out) {
     Vec3 a = v0 - r.org, b = v1 - r.org, c = v2 - r.org;
     float U, V, W, az, bz, cz;
     edge_functions(r, a, b, c, &U, &V, &W, &az, &bz, &cz);
@@ -459,21 +459,10 @@ SOL_HD bool intersect_triangle_upto(const RayShear& r, Vec3 v0, Vec3 v1, Vec3 v2
     float T = U * az + V * bz + W * cz;
     float rcp = 1.0f / det;
     float t = T * rcp;
-    if (!(t > tmin && t <= tmax)) return false;
+    if (!(t > tmin && t < tmax)) return false;
     *t_out = t;
     *u_out = V * rcp;
     *v_out = W * rcp;
-    return true;
-}
-
-/// intersect_triangle_upto for hits strictly inside (tmin, tmax).
-SOL_HD bool intersect_triangle(const RayShear& r, Vec3 v0, Vec3 v1, Vec3 v2,
-                               float tmin, float tmax, float* t_out, float* u_out, float* v_out) {
-    float t, u, v;
-    if (!intersect_triangle_upto(r, v0, v1, v2, tmin, tmax, &t, &u, &v) || !(t < tmax)) return false;
-    *t_out = t;
-    *u_out = u;
-    *v_out = v;
     return true;
 }
 
@@ -496,19 +485,6 @@ SOL_HD Vec3 safe_inverse(Vec3 d) {
     float y = fabs_(d.y) > eps ? d.y : copysign_(eps, d.y);
     float z = fabs_(d.z) > eps ? d.z : copysign_(eps, d.z);
     return vec3(1.0f / x, 1.0f / y, 1.0f / z);
-}
-
-/// Whether boxes stored as centre and half size (DBoxNode) may be tested along
-/// direction d.  The range keeps every quotient of a distance of at most 2e13 (the
-/// largest stored box) and a component finite, and those of scenes down to 1e-15
-/// out of the subnormal numbers.  A component below 2^-32 of the largest (zero
-/// above all) leaves the ray in a face of a box all along where its origin lies in
-/// it, and whether that is inside is decided by the last bit of the face, which
-/// a centre and a half size do not hold.
-SOL_HD bool boxes_take(Vec3 d) {
-    const float x = fabs_(d.x), y = fabs_(d.y), z = fabs_(d.z);
-    const float least = fminf(fminf(x, y), z), most = fmaxf(fmaxf(x, y), z);
-    return least >= 0x1p-32f * most && most >= 0x1p-47f && most <= 0x1p50f;
 }
 
 /// Widening factor applied to the exit distance of every slab test so that

@@ -15,8 +15,7 @@ struct SolGpuScene {
     int device = 0;
     int num_sms = 0;
     cudaStream_t stream = nullptr;
-    sol_b200::DBoxNode* boxes = nullptr;   // box nodes, then the nodes they were made from
-    sol_b200::DNode* nodes = nullptr;      // the second half of `boxes`
+    sol_b200::DNode* nodes = nullptr;
     sol_b200::DTri* tris = nullptr;
     sol_b200::DTriShade* shade = nullptr;
     char* tables = nullptr;          // one allocation: bsdfs, textures, images, lights, param_offsets, counters, fault

@@ -618,48 +618,10 @@ __global__ void gather_tris(const uint32_t* __restrict__ order, const int* __res
     }
 }
 
-/// Largest coordinate and half size of a packed box; larger (or non-finite)
-/// boxes are stored as boundless, which never culls.
-constexpr float kBoxRange = 1e13f;
-
-/// Centre and half size of one child's bounds on one axis.  The half size is
-/// measured from the rounded centre, rounded up, and enlarged by 16 units of
-/// 2^-24 for the rounding of child_boxes.
-__device__ __forceinline__ void pack_axis(float lo, float hi, float& centre, float& half) {
-    centre = 0.5f * lo + 0.5f * hi;
-    half = __fmul_ru(fmaxf(__fsub_ru(hi, centre), __fsub_ru(centre, lo)), 1.0f + 16.0f / 16777216.0f);
-    if (!(fabsf(centre) + half <= kBoxRange)) {
-        centre = 0.0f;
-        half = __int_as_float(0x7f800000);
-    }
-}
-
-__global__ void __launch_bounds__(256) pack_boxes(const DNode* __restrict__ nodes, uint32_t n, DBoxNode* __restrict__ boxes) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const DNode g = nodes[i];
-        DBoxNode b;
-        pack_axis(g.b0[0], g.b0[1], b.x[0], b.x[2]);
-        pack_axis(g.b1[0], g.b1[1], b.x[1], b.x[3]);
-        pack_axis(g.b0[2], g.b0[3], b.y[0], b.y[2]);
-        pack_axis(g.b1[2], g.b1[3], b.y[1], b.y[3]);
-        pack_axis(g.b2[0], g.b2[1], b.z[0], b.z[2]);
-        pack_axis(g.b2[2], g.b2[3], b.z[1], b.z[3]);
-        for (int k = 0; k < 4; ++k) b.ref[k] = g.ref[k];
-        boxes[i] = b;
-    }
-}
-
 template <typename T>
 cudaError_t alloc(T** p, size_t n) { return cudaMalloc(reinterpret_cast<void**>(p), sizeof(T) * (n ? n : 1)); }
 
 }  // namespace
-
-cudaError_t launch_pack_boxes(const DNode* nodes, uint32_t n, DBoxNode* boxes, cudaStream_t stream) {
-    if (n == 0) return cudaSuccess;
-    const int grid = (int)std::min<uint32_t>((n + 255) / 256, 8192);
-    pack_boxes<<<grid, 256, 0, stream>>>(nodes, n, boxes);
-    return cudaGetLastError();
-}
 
 cudaError_t build_lbvh(const float* vertices, const uint32_t* indices, const float* normals, const float* uvs,
                        const int32_t* tri_bsdf, const int32_t* tri_light, uint32_t num_triangles,
@@ -702,9 +664,7 @@ cudaError_t build_lbvh(const float* vertices, const uint32_t* indices, const flo
     layout();
     if (e == cudaSuccess) e = cudaMalloc(&work, work_bytes);
     if (e == cudaSuccess) layout();
-    static_assert(sizeof(DBoxNode) == sizeof(DNode), "both halves of the node allocation");
-    if (e == cudaSuccess) e = alloc(&out->boxes, 2 * (size_t)(n - 1));
-    if (e == cudaSuccess) out->nodes = reinterpret_cast<DNode*>(out->boxes + (n - 1));
+    if (e == cudaSuccess) e = alloc(&out->nodes, n - 1);
     if (e == cudaSuccess) e = alloc(&out->tris, n);
     if (e == cudaSuccess) e = alloc(&out->shade, n);
     const uint32_t init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
@@ -726,7 +686,6 @@ cudaError_t build_lbvh(const float* vertices, const uint32_t* indices, const flo
     }
     if (e == cudaSuccess) { tri_positions<<<grid, 256, 0, stream>>>(t, n, tri_pos); e = cudaGetLastError(); }
     if (e == cudaSuccess) { emit_nodes<<<grid, 256, 0, stream>>>(t, n, tri_pos, out->nodes); e = cudaGetLastError(); }
-    if (e == cudaSuccess) e = launch_pack_boxes(out->nodes, (uint32_t)(n - 1), out->boxes, stream);
     if (e == cudaSuccess) { node_depth<<<grid, 256, 0, stream>>>(t, n, depth); e = cudaGetLastError(); }
     if (e == cudaSuccess) { gather_tris<<<grid, 256, 0, stream>>>(order_sorted, tri_pos, num_triangles, vertices, normals, uvs, indices, tri_bsdf, tri_light, out->tris, out->shade); e = cudaGetLastError(); }
     unsigned int d = 0, failed = 0;
@@ -740,7 +699,7 @@ cudaError_t build_lbvh(const float* vertices, const uint32_t* indices, const flo
     cudaFree(work);
     if (e == cudaSuccess && failed) e = cudaErrorUnknown;   // a bottom-up walk did not reach the root
     if (e != cudaSuccess) {
-        cudaFree(out->boxes); cudaFree(out->tris); cudaFree(out->shade);
+        cudaFree(out->nodes); cudaFree(out->tris); cudaFree(out->shade);
         *out = LbvhResult{};
         return e;
     }

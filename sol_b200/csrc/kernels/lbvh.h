@@ -10,7 +10,6 @@ namespace sol_b200 {
 
 /// Device arrays of a built hierarchy, owned by the caller afterwards.
 struct LbvhResult {
-    DBoxNode* boxes = nullptr;     // num_nodes box nodes followed by `nodes`, one allocation
     DNode* nodes = nullptr;        // num_nodes entries, node 0 the root (unused entries zeroed)
     DTri* tris = nullptr;          // num_triangles, leaf order
     DTriShade* shade = nullptr;    // num_triangles, leaf order
@@ -18,9 +17,6 @@ struct LbvhResult {
     uint32_t depth = 0;            // node levels including the leaf level
     float sah_cost = 0.0f;         // SAH cost (traversal 1, triangle 1) normalised by the root's area
 };
-
-/// Box nodes (centre and half size) of `n` nodes, conservative for child_boxes.
-cudaError_t launch_pack_boxes(const DNode* nodes, uint32_t n, DBoxNode* boxes, cudaStream_t stream);
 
 /// Builds the hierarchy on the device from device arrays (vertices 3*nv floats,
 /// indices 3*nt, normals 3*nv, uvs 2*nv, per-triangle BSDF and light ids).

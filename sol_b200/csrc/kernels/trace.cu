@@ -15,17 +15,14 @@ namespace {
 /// a batch that the resident warps could hold with fewer lanes is spread over
 /// them, since the rays of a warp mostly trace one after another (1,000 closest
 /// hits 19.3 -> 14.3 us; from 8 lanes on the longest ray alone decides, 20,000
-/// take 36.9 us with 32 and 37.4 with 8).  `nodes` is s.nodes(), as a kernel parameter of its own
-/// so that the exact form's node addresses stay constant operands (1.5M shadow
-/// rays 133.1 -> 130.3 us).  64-thread blocks leave the SM as soon as their own
-/// longest ray ends; the occupancies (16 blocks: 64 registers, 24: 40) are the
-/// fastest measured: closest hits of 300k rays 38.8 us against 43.0 at 24 and
-/// 47.1 at 32 blocks, shadow rays 124.3 us against 125.6 at 16 and 131.6 at 32;
-/// 128-thread blocks 38.9 and 125.6.
+/// take 36.9 us with 32 and 37.4 with 8).  64-thread blocks leave the SM as soon
+/// as their own longest ray ends; the occupancies (16 blocks: 64 registers, 24:
+/// 40) are the fastest measured: closest hits of 300k rays 38.8 us against 43.0 at
+/// 24 and 47.1 at 32 blocks, shadow rays 124.3 us against 125.6 at 16 and 131.6
+/// at 32; 128-thread blocks 38.9 and 125.6.
 template <bool kAnyHit>
 __global__ void __launch_bounds__(kTraceBlock, kAnyHit ? 24 : 16)
-trace_rays(SceneView s, const DNode* __restrict__ nodes, const SolGpuRay* __restrict__ rays, uint32_t count,
-           SolGpuHit* __restrict__ hits, uint32_t lanes) {
+trace_rays(SceneView s, const SolGpuRay* __restrict__ rays, uint32_t count, SolGpuHit* __restrict__ hits, uint32_t lanes) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t i = (blockIdx.x * (kTraceBlock / 32u) + (threadIdx.x >> 5)) * lanes + lane;
     if (lane >= lanes || i >= count) return;
@@ -33,13 +30,10 @@ trace_rays(SceneView s, const DNode* __restrict__ nodes, const SolGpuRay* __rest
     const float4 b = __ldg(reinterpret_cast<const float4*>(rays + i) + 1);
     const Vec3 org = vec3(a.x, a.y, a.z), dir = vec3(b.x, b.y, b.z);
     TraversalCounters tc{0u, 0u};
-    // Any hit: which of several blockers is reported follows the host's order
-    // (the exact form), as the closest hit does.
     LocalStack stack;
-    Traversal<kAnyHit, false, false, kAnyHit> tr;
+    Traversal<kAnyHit, false, false> tr;   // in order, so that which of several blockers is reported is the host's choice
     tr.start(org, dir, a.w, b.w, s.num_tris > 0, stack);
-    tr.run(nodes, s.boxes, s.tris, tc, s.num_nodes, s.num_tris, s.max_steps, s.fault, stack, 0);
-    tr.resolve(s, b.w);
+    tr.run(s.nodes, s.tris, tc, s.num_nodes, s.num_tris, s.max_steps, s.fault, stack, 0);
     SolGpuHit h;
     h.tri = -1; h.t = 0.0f; h.u = 0.0f; h.v = 0.0f;
     if (tr.hit >= 0) {
@@ -61,8 +55,8 @@ cudaError_t launch_trace(const SceneView& s, const SolGpuRay* rays, uint32_t cou
     if (lanes > 4u) lanes = 32;
     const uint32_t per_block = lanes * (kTraceBlock / 32);
     const uint32_t grid = (uint32_t)(((uint64_t)count + per_block - 1) / per_block);
-    if (any_hit) trace_rays<true><<<grid, kTraceBlock, 0, stream>>>(s, s.nodes(), rays, count, hits, lanes);
-    else trace_rays<false><<<grid, kTraceBlock, 0, stream>>>(s, s.nodes(), rays, count, hits, lanes);
+    if (any_hit) trace_rays<true><<<grid, kTraceBlock, 0, stream>>>(s, rays, count, hits, lanes);
+    else trace_rays<false><<<grid, kTraceBlock, 0, stream>>>(s, rays, count, hits, lanes);
     return cudaGetLastError();
 }
 

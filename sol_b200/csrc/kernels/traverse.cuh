@@ -2,24 +2,21 @@
 // TriangleMesh::intersect_closest / intersect_any (src/triangle_mesh.cpp:64-117),
 // which SoL runs through bvh v2's SingleRayTraverser.
 //
-// The traversal is the stack-based "while-while" loop of Aila & Laine
-// ("Understanding the Efficiency of Ray Traversal on GPUs", HPG 2009): descend
-// inner nodes, pushing the child that waits, until a leaf is reached; then test
-// the leaf's triangles (48 bytes, three 128-bit loads) with the shared watertight
-// test, so a hit found here is bit-identical to the one the host finds.
-//
-// Two forms of the box test walk the same hierarchy:
-//   exact  (DNode, lower and upper bounds): the host traversal's operations, so
-//          children are visited in the host's order and the first of several hits
-//          is the host's.  Ray queries for any hit, which return that hit, and the
-//          counting kernels use it.
-//   packed (DBoxNode, centre and half size): fewer operations, conservative too,
-//          in an order that may differ from the host's where two boxes begin at
-//          (nearly) equal distances.  The closest hit is the same unless several
-//          triangles are hit at exactly the closest distance; a ray that meets
-//          that case is traced again in the exact form (closest_exact), and so is
-//          one whose direction the packed test does not take (boxes_take).  A
-//          shadow ray only asks whether anything is hit, which no order changes.
+// Layout: every inner node is 64 bytes holding both child boxes, fetched in two
+// 256-bit read-only loads; triangles are 48 bytes (three 128-bit loads).  The
+// traversal is the stack-based "while-while" loop of Aila & Laine ("Understanding
+// the Efficiency of Ray Traversal on GPUs", HPG 2009): descend inner nodes
+// nearest-child first, pushing the farther child, until a leaf is reached; then
+// test the leaf's triangles.  Box tests compute (bound - origin) / direction and
+// widen the exit distance by kSlabWiden so that they are conservative; they are
+// the same operations as the host traversal's, so both visit children in the same
+// order and resolve equal-distance hits alike.  The triangle test is the shared
+// watertight test, so a hit found here is bit-identical to the one the host finds.
+// (Boxes stored as centre and half size need 12 fewer operations per node: frame
+// 46.1 -> 43.7 ms, Cornell box 1414 -> 1351 us.  But they have to be enlarged for
+// their rounding, which changes which boxes count as entered at their faces: with
+// coordinates of 1000 and more and a ray offset of 1e-5, up to 0.04 % of the
+// bounces then hit the surface that they leave, whose box the host culls.)
 #pragma once
 
 #include "../core/layout.h"
@@ -122,82 +119,24 @@ __device__ __forceinline__ void child_slabs(float4 a, float4 b, float4 c, Vec3 o
     f1 = fminf3(fmaxf(t1lx, t1hx), fmaxf(t1ly, t1hy), fminf(fmaxf(t1lz, t1hz), tmax)) * kSlabWiden;
 }
 
-/// Two floats as one packed register pair operand.
-struct F2 { float a, b; };
-__device__ __forceinline__ F2 sub2(F2 x, float y) {
-    F2 r;
-    asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %4};\n\tsub.rn.f32x2 p, p, q;\n\t"
-        "mov.b64 {%0, %1}, p;\n\t}" : "=f"(r.a), "=f"(r.b) : "f"(x.a), "f"(x.b), "f"(y));
-    return r;
-}
-__device__ __forceinline__ F2 mul2(F2 x, float y) {
-    F2 r;
-    asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %4};\n\tmul.rn.f32x2 p, p, q;\n\t"
-        "mov.b64 {%0, %1}, p;\n\t}" : "=f"(r.a), "=f"(r.b) : "f"(x.a), "f"(x.b), "f"(y));
-    return r;
-}
-__device__ __forceinline__ F2 fma2(F2 x, float y, F2 z) {
-    F2 r;
-    asm("{\n\t.reg .b64 p, q, s;\n\tmov.b64 p, {%2, %3};\n\tmov.b64 q, {%4, %4};\n\tmov.b64 s, {%5, %6};\n\t"
-        "fma.rn.f32x2 p, p, q, s;\n\tmov.b64 {%0, %1}, p;\n\t}"
-        : "=f"(r.a), "=f"(r.b) : "f"(x.a), "f"(x.b), "f"(y), "f"(z.a), "f"(z.b));
-    return r;
-}
-
-/// child_slabs on a DBoxNode: per axis both children's centre distances
-/// (c - o) / d in one packed subtract and multiply, then entry and exit as
-/// that distance -+ h |1/d| in two packed fused multiply-adds: 12 packed
-/// operations for both boxes, and no minimum or maximum to order the planes
-/// (the exact form has 12 of each).  Node steps are issue-bound, so this shows
-/// in full: 1M-triangle frame, 64 samples 46.5 -> 43.8 ms, Cornell box 1409 ->
-/// 1357 us, 300k closest-hit rays 42.9 -> 39.2 us (with the two 32-byte loads,
-/// of which the frame's share is 0.8 ms).
-///
-/// Conservative: with eps = 2^-24, D = |c - o| / |d| and H = h / |d|, either
-/// distance errs by at most (3 D + H + |distance|) eps (subtraction, 1/d and
-/// multiplication on the first term, 1/d on the second, the sum's rounding).
-/// pack_boxes enlarges h by 16 eps, which covers D <= H; beyond, |distance| <=
-/// D + H and half of the exit's widening (13 eps in all) of a distance of at
-/// least D - H covers the rest, since 16 + 6.5 (D / H - 1) >= 4 D / H + 2, with
-/// at least 2.5 D eps to spare for the triangle test's own rounding.  (The
-/// approximate reciprocal errs by 2 eps, which takes 1 D of that; it gained 1 %
-/// on the frame.)
-__device__ __forceinline__ void child_boxes(float4 x, float4 y, float4 z, Vec3 org, Vec3 idir, float tmin, float tmax,
-                                            float& n0, float& f0, float& n1, float& f1) {
-    const float ax = fabsf(idir.x), ay = fabsf(idir.y), az = fabsf(idir.z);
-    const F2 cx = mul2(sub2(F2{x.x, x.y}, org.x), idir.x), hx{x.z, x.w};
-    const F2 cy = mul2(sub2(F2{y.x, y.y}, org.y), idir.y), hy{y.z, y.w};
-    const F2 cz = mul2(sub2(F2{z.x, z.y}, org.z), idir.z), hz{z.z, z.w};
-    const F2 nx = fma2(hx, -ax, cx), ny = fma2(hy, -ay, cy), nz = fma2(hz, -az, cz);
-    const F2 fx = fma2(hx, ax, cx), fy = fma2(hy, ay, cy), fz = fma2(hz, az, cz);
-    n0 = fmaxf3(nx.a, ny.a, fmaxf(nz.a, tmin));
-    n1 = fmaxf3(nx.b, ny.b, fmaxf(nz.b, tmin));
-    f0 = fminf3(fx.a, fy.a, fminf(fz.a, tmax)) * kSlabWiden;
-    f1 = fminf3(fx.b, fy.b, fminf(fz.b, tmax)) * kSlabWiden;
-}
-
-/// A box node in two 32-byte loads.
-__device__ __forceinline__ void load_boxes(const DBoxNode* n, float4& x, float4& y, float4& z, int2& ref) {
+/// A node in two 32-byte loads (four of 16 bytes: frame 48.0 against 46.1 ms,
+/// Cornell box 1465 against 1414 us).
+__device__ __forceinline__ void load_node(const DNode* n, float4& a, float4& b, float4& c, int2& ref) {
     asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w), "=f"(y.x), "=f"(y.y), "=f"(y.z), "=f"(y.w) : "l"(n));
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(n));
     asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, _, _}, [%6 + 32];"
-        : "=f"(z.x), "=f"(z.y), "=f"(z.z), "=f"(z.w), "=r"(ref.x), "=r"(ref.y) : "l"(n));
+        : "=f"(c.x), "=f"(c.y), "=f"(c.z), "=f"(c.w), "=r"(ref.x), "=r"(ref.y) : "l"(n));
 }
-
-/// Set in Traversal::hit when the exact traversal has to find the hit: another
-/// triangle was hit at exactly the distance of the closest one (positions in
-/// leaf order stay below 2^28), or the direction is none that boxes_take.
-constexpr int kRedoBit = 1 << 30;
 
 /// BVH traversal of one ray as a resumable state: start() sets it up, run()
 /// advances it.  For kAnyHit the first triangle hit inside (tmin, tmax) is
 /// kept; otherwise the closest one, with `tmax` shrunk to its distance.  `hit`
-/// is the triangle's position in leaf order, or -1.  A packed traversal
-/// (kExact = false) must be followed by resolve().
+/// is the triangle's position in leaf order, or -1.
 ///
-/// A packed any-hit traversal takes the first child first, whichever is nearer:
-/// the answer does not depend on the order, and not ordering the children saves
-/// more than it costs (frame 47.0 -> 46.2 ms, 24-view batch 9.87 -> 9.49 ms).
+/// Without kOrdered (any-hit only) the first child is taken first, whichever is
+/// nearer.  Which of several hits is found follows the order, whether there is
+/// one does not, and not ordering the children saves more than it costs (frame
+/// 47.0 -> 46.2 ms, 24-view batch 9.87 -> 9.49 ms).
 ///
 /// With kYield, run() may return early, after a leaf, when fewer than
 /// `min_active` lanes of the warp are still traversing: the caller gives the
@@ -210,8 +149,9 @@ constexpr int kRedoBit = 1 << 30;
 /// Self-checks: at most `max_steps` steps, node and triangle references checked
 /// against the array sizes and the stack against its capacity; a failed check
 /// ORs a kFault* bit into `*fault` and ends the traversal with no hit.
-template <bool kAnyHit, bool kCount, bool kYield, bool kExact>
+template <bool kAnyHit, bool kCount, bool kYield, bool kOrdered = true>
 struct Traversal {
+    static_assert(kAnyHit || kOrdered, "a closest hit needs the nearer child first");
     Vec3 org, dir, idir;
     RayShear rs;
     float tmin, tmax;
@@ -225,7 +165,7 @@ struct Traversal {
         dir = d;
         tmin = t0;
         tmax = t1;
-        idir = kExact ? safe_inverse(d) : vec3(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);   // the same where boxes_take(d)
+        idir = safe_inverse(d);
         rs = make_shear(o, d);
         sp = 0;
         hit = -1;
@@ -233,10 +173,6 @@ struct Traversal {
         steps = 0;
         node = active ? 0 : kStackSentinel;
         stack.put(sp++, kStackSentinel);
-        if (!kExact && active && !boxes_take(d)) {   // nothing to run, resolve() traces the ray
-            node = kStackSentinel;
-            hit = kRedoBit;
-        }
     }
 
     __device__ __forceinline__ bool fail(unsigned int* fault, unsigned int bit) {
@@ -246,13 +182,11 @@ struct Traversal {
         return true;
     }
 
-    /// Advances the traversal; true when it has finished.  `exact_nodes` is
-    /// used by the exact form, `boxes` by the packed one.
+    /// Advances the traversal; true when it has finished.
     template <class Stack>
-    __device__ __forceinline__ bool run(const DNode* __restrict__ exact_nodes, const DBoxNode* __restrict__ boxes,
-                                        const DTri* __restrict__ tris, TraversalCounters& ctr, uint32_t num_nodes,
-                                        uint32_t num_tris, uint32_t max_steps, unsigned int* fault, Stack& stack,
-                                        int min_active) {
+    __device__ __forceinline__ bool run(const DNode* __restrict__ nodes, const DTri* __restrict__ tris,
+                                        TraversalCounters& ctr, uint32_t num_nodes, uint32_t num_tris,
+                                        uint32_t max_steps, unsigned int* fault, Stack& stack, int min_active) {
         while (node != kStackSentinel) {
             // Descend inner nodes until a leaf, the end or a reference outside the
             // node array is reached: as unsigned numbers leaf references and the
@@ -260,25 +194,15 @@ struct Traversal {
             while ((uint32_t)node < num_nodes) {
                 if (++steps > max_steps) return fail(fault, kFaultTraversalSteps);
                 if (kCount) ctr.nodes++;
-                float n0, f0, n1, f1;
+                float4 a, b, c;
                 int2 r;
-                if (kExact) {
-                    const DNode* n = exact_nodes + node;
-                    const float4 a = ldg4(n->b0);
-                    const float4 b = ldg4(n->b1);
-                    const float4 c = ldg4(n->b2);
-                    const int4 r4 = __ldg(reinterpret_cast<const int4*>(n->ref));
-                    r = make_int2(r4.x, r4.y);
-                    child_slabs(a, b, c, org, idir, tmin, tmax, n0, f0, n1, f1);
-                } else {
-                    float4 x, y, z;
-                    load_boxes(boxes + node, x, y, z, r);
-                    child_boxes(x, y, z, org, idir, tmin, tmax, n0, f0, n1, f1);
-                }
+                load_node(nodes + node, a, b, c, r);
+                float n0, f0, n1, f1;
+                child_slabs(a, b, c, org, idir, tmin, tmax, n0, f0, n1, f1);
                 const bool h0 = n0 <= f0, h1 = n1 <= f1;
                 if (h0 && h1) {
                     int near = r.x, far = r.y;
-                    if ((kExact || !kAnyHit) && n1 < n0) { near = r.y; far = r.x; }
+                    if (kOrdered && n1 < n0) { near = r.y; far = r.x; }
                     if (sp >= kTraversalStack) return fail(fault, kFaultTraversalSteps);
                     stack.put(sp++, far);
                     node = near;
@@ -303,26 +227,12 @@ struct Traversal {
                 const float4 p0 = ldg4(tp->v0), p1 = ldg4(tp->v1), p2 = ldg4(tp->v2);
                 if (kCount) ctr.tris++;
                 float t, u, w;
-                if (kAnyHit || kExact) {
-                    if (intersect_triangle(rs, tri_vertex(p0), tri_vertex(p1), tri_vertex(p2), tmin, tmax, &t, &u, &w)) {
-                        hit = (int)i;
-                        tmax = t;
-                        if (kAnyHit) break;
-                        hu = u;
-                        hv = w;
-                    }
-                } else if (intersect_triangle_upto(rs, tri_vertex(p0), tri_vertex(p1), tri_vertex(p2), tmin, tmax, &t,
-                                                   &u, &w)) {
-                    if (t < tmax) {
-                        hit = (int)i;
-                        tmax = t;
-                        hu = u;
-                        hv = w;
-                    } else if (hit >= 0 && (hit & ~kRedoBit) != (int)i) {
-                        // (Without a hit, tmax is the ray's own end, which is no hit; a tree of
-                        // one leaf has it as both children of its root.)
-                        hit |= kRedoBit;
-                    }
+                if (intersect_triangle(rs, tri_vertex(p0), tri_vertex(p1), tri_vertex(p2), tmin, tmax, &t, &u, &w)) {
+                    hit = (int)i;
+                    tmax = t;
+                    if (kAnyHit) break;
+                    hu = u;
+                    hv = w;
                 }
             }
             if (kAnyHit && hit >= 0) return true;
@@ -332,67 +242,31 @@ struct Traversal {
         }
         return true;
     }
-
-    /// After a packed traversal that began with the end `t1`: where kRedoBit is
-    /// set, the hit that the exact traversal finds.
-    __device__ __forceinline__ void resolve(const SceneView& s, float t1);
 };
 
-/// The closest hit of one ray by the exact traversal, out of line: only the few
-/// rays with kRedoBit come here.  (Whether there is any hit is the same question
-/// for both queries: they part only after the first.)
-struct ExactHit { int hit; float t, u, v; };
-static __device__ __noinline__ ExactHit closest_exact(const DNode* nodes, const DTri* tris, uint32_t num_nodes,
-                                                      uint32_t num_tris, uint32_t max_steps, unsigned int* fault,
-                                                      Vec3 org, Vec3 dir, float tmin, float tmax) {
-    LocalStack stack;
-    TraversalCounters tc{0u, 0u};
-    Traversal<false, false, false, true> tr;
-    tr.start(org, dir, tmin, tmax, true, stack);
-    tr.run(nodes, nullptr, tris, tc, num_nodes, num_tris, max_steps, fault, stack, 0);
-    return ExactHit{tr.hit, tr.tmax, tr.hu, tr.hv};
-}
-
-template <bool kAnyHit, bool kCount, bool kYield, bool kExact>
-__device__ __forceinline__ void Traversal<kAnyHit, kCount, kYield, kExact>::resolve(const SceneView& s, float t1) {
-    if (kExact || hit < kRedoBit) return;
-    const ExactHit e = closest_exact(s.nodes(), s.tris, s.num_nodes, s.num_tris, s.max_steps, s.fault, org, dir, tmin, t1);
-    hit = e.hit;
-    tmax = e.t;
-    hu = e.u;
-    hv = e.v;
-}
-
-/// Traverses a scene's BVH for one ray to completion (see Traversal).  Returns
-/// the hit triangle's position in leaf order, or -1; `tmax` becomes the hit
-/// distance, (u, v) the barycentrics of a closest hit.
-template <bool kAnyHit, bool kCount, bool kExact, class Stack>
-__device__ __forceinline__ int traverse_uv(const SceneView& s, Vec3 org, Vec3 dir, float tmin, float& tmax, float& u,
-                                           float& v, TraversalCounters& ctr, Stack& stack) {
-    Traversal<kAnyHit, kCount, false, kExact> tr;
-    const float t1 = tmax;
+/// Closest hit of one ray of a scene.  Returns the hit triangle's position in leaf
+/// order, or -1; `tmax` becomes the hit distance, (u, v) its barycentrics.
+template <bool kCount, class Stack>
+__device__ __forceinline__ int traverse_closest_uv(const SceneView& s, Vec3 org, Vec3 dir, float tmin, float& tmax,
+                                                   float& u, float& v, TraversalCounters& ctr, Stack& stack) {
+    Traversal<false, kCount, false> tr;
     tr.start(org, dir, tmin, tmax, s.num_tris > 0, stack);
-    tr.run(s.nodes(), s.boxes, s.tris, ctr, s.num_nodes, s.num_tris, s.max_steps, s.fault, stack, 0);
-    tr.resolve(s, t1);
+    tr.run(s.nodes, s.tris, ctr, s.num_nodes, s.num_tris, s.max_steps, s.fault, stack, 0);
     tmax = tr.tmax;
     u = tr.hu;
     v = tr.hv;
     return tr.hit;
 }
 
-/// Closest hit for the render kernels (the counting ones walk the exact form).
-template <bool kCount, class Stack>
-__device__ __forceinline__ int traverse_closest_uv(const SceneView& s, Vec3 org, Vec3 dir, float tmin, float& tmax,
-                                                   float& u, float& v, TraversalCounters& ctr, Stack& stack) {
-    return traverse_uv<false, kCount, kCount>(s, org, dir, tmin, tmax, u, v, ctr, stack);
-}
-
-/// Whether a shadow ray is blocked before `tmax`.
+/// Whether a shadow ray is blocked before `tmax`.  The counting kernels take the
+/// host's order, so that they count what the host visits.
 template <bool kCount, class Stack>
 __device__ __forceinline__ bool occluded(const SceneView& s, Vec3 org, Vec3 dir, float tmin, float tmax,
                                          TraversalCounters& ctr, Stack& stack) {
-    float u, v;
-    return traverse_uv<true, kCount, kCount>(s, org, dir, tmin, tmax, u, v, ctr, stack) >= 0;
+    Traversal<true, kCount, false, kCount> tr;
+    tr.start(org, dir, tmin, tmax, s.num_tris > 0, stack);
+    tr.run(s.nodes, s.tris, ctr, s.num_nodes, s.num_tris, s.max_steps, s.fault, stack, 0);
+    return tr.hit >= 0;
 }
 
 }  // namespace sol_b200

@@ -249,7 +249,7 @@ using WfStack = LocalStack;
 __device__ __forceinline__ WfStack make_stack() { return WfStack{}; }
 #endif
 
-/// Traces the `n` rays of a queue, which end at `t1`.  When the launch's warps could hold them all
+/// Traces the `n` rays of a queue.  When the launch's warps could hold them all
 /// with fewer, only that many lanes of each warp (a power of two) take rays: the
 /// last bounces of a batch leave a few thousand incoherent rays, which a warp
 /// of 32 traces nearly one after another (24 views, bounces 10 to 16: 120-200
@@ -257,9 +257,9 @@ __device__ __forceinline__ WfStack make_stack() { return WfStack{}; }
 /// 0.69 ms, twenty single-sample views 1.06 -> 0.93 ms).
 template <bool kAnyHit, class Fetch, class Finish>
 __device__ __forceinline__ void trace_queue(const WfSceneTable& scenes, uint32_t n, uint32_t* fetch_counter,
-                                            int refill_below, float t1, Fetch fetch, Finish finish,
+                                            int refill_below, Fetch fetch, Finish finish,
                                             unsigned long long& rays) {
-    Traversal<kAnyHit, false, true, false> tr;
+    Traversal<kAnyHit, false, true, !kAnyHit> tr;
     WfStack stack = make_stack();
     const SceneView* sv = &scenes.v[0];
     uint32_t at = 0;
@@ -294,9 +294,8 @@ __device__ __forceinline__ void trace_queue(const WfSceneTable& scenes, uint32_t
         }
         if (!__any_sync(0xffffffffu, has)) break;
         // Once the queue is drained there is nothing to refill: run to the end.
-        if (has && tr.run(nullptr, sv->boxes, sv->tris, tc, sv->num_nodes, sv->num_tris, sv->max_steps, sv->fault,
-                          stack, more ? refill_below : 0)) {
-            tr.resolve(*sv, t1);
+        if (has && tr.run(sv->nodes, sv->tris, tc, sv->num_nodes, sv->num_tris, sv->max_steps, sv->fault, stack,
+                          more ? refill_below : 0)) {
             finish(at, tr);
             has = false;
         }
@@ -316,13 +315,13 @@ wf_extend(const WfParams* __restrict__ Pp, const __grid_constant__ WfSceneTable 
     const float4* __restrict__ ro = P.ray_o[p];
     const float4* __restrict__ rd = P.ray_d[p];
     unsigned long long rays = 0;
-    auto fetch = [&](uint32_t i, Traversal<false, false, true, false>& tr, WfStack& stack) -> uint32_t {
+    auto fetch = [&](uint32_t i, Traversal<false, false, true>& tr, WfStack& stack) -> uint32_t {
         const float4 o = ro[i], d = rd[i];
         const uint32_t scene = __float_as_uint(d.w) >> kWfSlotBits;
         tr.start(vec3(o.x, o.y, o.z), vec3(d.x, d.y, d.z), o.w, kFloatMax, scenes.v[scene].num_tris > 0, stack);
         return scene;
     };
-    auto finish = [&](uint32_t i, const Traversal<false, false, true, false>& tr) {
+    auto finish = [&](uint32_t i, const Traversal<false, false, true>& tr) {
         P.hit[i] = make_float4(__int_as_float(tr.hit), tr.tmax, tr.hu, tr.hv);
         if (sort) {
             int kind = kWfBins - 1;
@@ -334,7 +333,7 @@ wf_extend(const WfParams* __restrict__ Pp, const __grid_constant__ WfSceneTable 
             P.q_bins[(size_t)kind * P.capacity + append_keyed(ctr->bins, kind)] = i;
         }
     };
-    trace_queue<false>(scenes, n, &ctr->fetch_extend, P.refill_below, kFloatMax, fetch, finish, rays);
+    trace_queue<false>(scenes, n, &ctr->fetch_extend, P.refill_below, fetch, finish, rays);
     rays = warp_sum(rays);
     if (lane_id() == 0 && rays) atomicAdd(&ctr->rays, rays);
 }
@@ -452,7 +451,7 @@ wf_shadow(const WfParams* __restrict__ Pp, const __grid_constant__ WfSceneTable 
         }
         if (P.sh_d[i].w != 0.0f) P.q_ended[q][append(&ctr->ended[q])] = slot;
     };
-    trace_queue<true>(scenes, n, &ctr->fetch_shadow, P.refill_below, 1.0f - offset, fetch, finish, rays);
+    trace_queue<true>(scenes, n, &ctr->fetch_shadow, P.refill_below, fetch, finish, rays);
     rays = warp_sum(rays);
     if (lane_id() == 0 && rays) { atomicAdd(&ctr->rays, rays); atomicAdd(&ctr->shadow_rays, rays); }
 }
