@@ -112,8 +112,9 @@ int render_into(SolGpuScene* scene, const SolGpuCamera* camera, const SolGpuConf
     // Split schedule (one work item per pixel sample, measured faster than the
     // per-pixel schedule on small and full-size frames alike) for every render
     // of more than one sample, in chunks of samples whose colours fit in the
-    // scratch limit; the per-pixel schedule for single samples, on request, or
-    // when not even one sample's colours fit.
+    // scratch limit; the per-pixel schedule on request or when not even one
+    // sample's colours fit.  A single sample needs no scratch: it goes into the
+    // film directly, one path per work item too.
     const uint64_t pixels = (uint64_t)width * height;
     const uint64_t sample_items = (uint64_t)((width + 7) / 8) * ((height + 3) / 4) * 32;
     const uint64_t sample_floats = 3 * pixels;
@@ -144,12 +145,12 @@ int render_into(SolGpuScene* scene, const SolGpuCamera* camera, const SolGpuConf
     }
     // One path per work item (lean): the full-occupancy build when there is
     // enough to trace for its resident lanes (kMegakernelFullVerticesPerLane).
-    const bool lean = split || sample_count == 1;
-    int per_sm = megakernel_blocks_per_sm(scene->instrumented, lean, true, basic);
+    const Megakernel kind = split ? Megakernel::kSplit : sample_count == 1 ? Megakernel::kSingle : Megakernel::kPerPixel;
+    int per_sm = megakernel_blocks_per_sm(kind, scene->instrumented, true, basic);
     const uint64_t vertices = pixels * (split ? chunk : 1) *
         std::min(std::max(config->max_path_len, kMegakernelMinCountedLen), kMegakernelMaxCountedLen);
     const bool full = vertices > kMegakernelFullVerticesPerLane * (uint64_t)per_sm * scene->num_sms * kMegakernelBlock;
-    if (lean && !full) per_sm = megakernel_blocks_per_sm(scene->instrumented, lean, false, basic);
+    if (kind != Megakernel::kPerPixel && !full) per_sm = megakernel_blocks_per_sm(kind, scene->instrumented, false, basic);
     if (per_sm <= 0) return fail(SOL_GPU_ERR_CUDA, "megakernel occupancy query failed");
     const int grid = per_sm * scene->num_sms;
     cudaEventRecord(scene->ev_start, stream);

@@ -71,12 +71,16 @@ struct L2Window {
     float hit_ratio = 1.0f;
 };
 
-/// Resident blocks per SM of the megakernel (for sizing its persistent grid);
-/// `lean`: the kernel of one path per work item (the split schedule and single
-/// samples), in its full-occupancy build (`full`, kMegakernelMinBlocks) or the
-/// kMegakernelSmallMinBlocks one; `basic`: the build without image textures
-/// and Interp BSDFs, for scenes that have neither (SolGpuScene::basic_shading).
-int megakernel_blocks_per_sm(bool instrumented, bool lean, bool full, bool basic);
+/// K1's kernels: one pixel per work item; one path per work item (the lean
+/// kernel), added into the film (a single sample) or written to scratch (split).
+enum class Megakernel { kPerPixel, kSingle, kSplit };
+
+/// Resident blocks per SM of the megakernel that such a render launches (for
+/// sizing its persistent grid).  `full`: the lean kernel's full-occupancy build
+/// (kMegakernelMinBlocks), else the kMegakernelSmallMinBlocks one; `basic`: the
+/// build without image textures and Interp BSDFs, for scenes that have neither
+/// (SolGpuScene::basic_shading).
+int megakernel_blocks_per_sm(Megakernel kind, bool instrumented, bool full, bool basic);
 
 /// K1: renders samples [sample_index, sample_index + sample_count) of every
 /// pixel and adds each pixel's sum into `film` (3 planes of width*height).

@@ -454,15 +454,15 @@ sum_samples_views(const WfView* __restrict__ views, uint32_t num_views, uint64_t
 
 namespace {
 
-/// The K1 instantiation for a schedule, occupancy target and shading (basic:
-/// the scene has no image textures and no Interp BSDFs; the counting build
-/// always has full shading).
-template <bool kSplit>
-auto megakernel_fn(bool instrumented, bool basic) {
-    if (instrumented) return pt_megakernel<true, kSplit, kMegakernelMinBlocks, false>;
-    return basic ? pt_megakernel<false, kSplit, kMegakernelMinBlocks, true>
-                 : pt_megakernel<false, kSplit, kMegakernelMinBlocks, false>;
+/// K1's instantiations (basic: the scene has no image textures and no Interp
+/// BSDFs; the counting builds always have full shading).  Split samples without
+/// counters run on the lean kernel only.
+auto per_pixel_fn(bool instrumented, bool basic) {
+    if (instrumented) return pt_megakernel<true, false, kMegakernelMinBlocks, false>;
+    return basic ? pt_megakernel<false, false, kMegakernelMinBlocks, true>
+                 : pt_megakernel<false, false, kMegakernelMinBlocks, false>;
 }
+auto counting_split_fn() { return pt_megakernel<true, true, kMegakernelMinBlocks, false>; }
 template <bool kFilm>
 auto lean_fn(bool full, bool basic) {
     if (basic) return full ? pt_megakernel_lean<kMegakernelMinBlocks, true, kFilm>
@@ -496,12 +496,14 @@ cudaError_t launch_lean(const SceneView& s, const DCamera& cam, const DConfig& c
 
 }  // namespace
 
-int megakernel_blocks_per_sm(bool instrumented, bool lean, bool full, bool basic) {
+int megakernel_blocks_per_sm(Megakernel kind, bool instrumented, bool full, bool basic) {
     int n = 0;
-    const cudaError_t e = lean && !instrumented
-        ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, lean_fn<false>(full, basic), kMegakernelBlock, 0)
-        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, megakernel_fn<true>(instrumented, basic), kMegakernelBlock, 0);
-    return e == cudaSuccess ? n : -1;
+    auto query = [&](auto fn) {
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kMegakernelBlock, 0) == cudaSuccess ? n : -1;
+    };
+    if (instrumented) return kind == Megakernel::kSplit ? query(counting_split_fn()) : query(per_pixel_fn(true, basic));
+    if (kind == Megakernel::kPerPixel) return query(per_pixel_fn(false, basic));
+    return kind == Megakernel::kSingle ? query(lean_fn<true>(full, basic)) : query(lean_fn<false>(full, basic));
 }
 
 cudaError_t launch_megakernel(const SceneView& s, const DCamera& cam, const DConfig& cfg,
@@ -510,7 +512,7 @@ cudaError_t launch_megakernel(const SceneView& s, const DCamera& cam, const DCon
                               int grid, cudaStream_t stream, const L2Window& l2) {
     if (!instrumented && sample_count == 1)
         return launch_lean<true>(s, cam, cfg, sample_index, 1, width, height, film, counters, full, basic, grid, stream, l2);
-    return launch_l2(megakernel_fn<false>(instrumented, basic), grid, kMegakernelBlock, 0, stream, l2, s, cam, cfg,
+    return launch_l2(per_pixel_fn(instrumented, basic), grid, kMegakernelBlock, 0, stream, l2, s, cam, cfg,
                      sample_index, sample_count, width, height, film, counters);
 }
 
@@ -557,7 +559,7 @@ cudaError_t launch_megakernel_split(const SceneView& s, const DCamera& cam, cons
         cudaError_t e = cudaSuccess;
         if (c0 > 0) e = cudaMemsetAsync(&counters->next_item, 0, sizeof(counters->next_item), stream);
         if (e != cudaSuccess) return e;
-        e = instrumented ? launch_l2(megakernel_fn<true>(true, basic), grid, kMegakernelBlock, 0, stream, l2, s, cam, cfg,
+        e = instrumented ? launch_l2(counting_split_fn(), grid, kMegakernelBlock, 0, stream, l2, s, cam, cfg,
                                      sample_index + c0, k, width, height, scratch, counters)
                          : launch_lean<false>(s, cam, cfg, sample_index + c0, k, width, height, scratch, counters, full,
                                               basic, grid, stream, l2);
