@@ -134,7 +134,7 @@ pt_megakernel(SceneView s, DCamera cam, DConfig cfg, uint64_t sample_index, uint
         VertexOut vo;
         vo.has_shadow = false;
         vo.end = slot < 0;
-        if (!vo.end) shade_vertex<kBasic ? kShadeBasic : kShadeFull>(s, cfg, light_pick_prob, slot, t, ps, vo, true, hu, hv);
+        if (!vo.end) shade_vertex<kBasic ? kShadeBasic : kShadeCall>(s, cfg, light_pick_prob, slot, t, ps, vo, true, hu, hv);
 
         // --- shadow ray of this vertex (path_tracer.cpp:72-74) -------------
         if (vo.has_shadow) {
@@ -238,7 +238,7 @@ pt_megakernel_lean(SceneView s, DCamera cam, DConfig cfg, uint64_t sample_index,
                     end = true;
                 } else {
                     VertexOut vo;
-                    shade_vertex<kBasic ? kShadeBasic : kShadeFull>(s, cfg, light_pick_prob, slot, t, ps, vo, true, hu, hv);
+                    shade_vertex<kBasic ? kShadeBasic : kShadeCall>(s, cfg, light_pick_prob, slot, t, ps, vo, true, hu, hv);
                     // shadow ray of this vertex (path_tracer.cpp:72-74)
                     if (vo.has_shadow) {
                         const bool occ =

@@ -36,10 +36,10 @@ namespace sol_b200 {
 // Textures (include/sol/textures.h:97-144, src/textures.cpp:5-52)
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ Rgb texel(const SceneView& s, const DImage& img, int x, int y) {
+__device__ __forceinline__ Rgb texel(const float* __restrict__ texels, const DImage& img, int x, int y) {
     size_t plane = (size_t)img.width * img.height;
     size_t i = img.offset + (size_t)y * img.width + (size_t)x;
-    return rgb(__ldg(s.texels + i), __ldg(s.texels + i + plane), __ldg(s.texels + i + 2 * plane));
+    return rgb(__ldg(texels + i), __ldg(texels + i + plane), __ldg(texels + i + 2 * plane));
 }
 
 __device__ __forceinline__ float fmod2_(float x) {
@@ -47,8 +47,11 @@ __device__ __forceinline__ float fmod2_(float x) {
     return fmodf(x, 2.0f);
 }
 
-/// ImageTexture<Filter, Border>::sample_color (src/textures.cpp:47-52).
-__device__ SOL_TEX_FN Rgb image_color(const SceneView& s, const DTexture& t, Vec2 uv) {
+/// ImageTexture<Filter, Border>::sample_color (src/textures.cpp:47-52).  It takes
+/// the two arrays and not the scene, whose address would put a copy of a kernel's
+/// scene parameter on every thread's stack where this is not inlined.
+__device__ SOL_TEX_FN Rgb image_color(const DImage* __restrict__ images, const float* __restrict__ texels,
+                                      const DTexture& t, Vec2 uv) {
     // Border handling (textures.cpp:5-21); Mirror uses uv[0] for both axes as SoL does.
     if (t.border == SOL_GPU_BORDER_CLAMP) {
         uv = vec2(clampf(uv.x, 0.0f, 1.0f), clampf(uv.y, 0.0f, 1.0f));
@@ -60,13 +63,13 @@ __device__ SOL_TEX_FN Rgb image_color(const SceneView& s, const DTexture& t, Vec
         v = v > 1.0f ? 2.0f - v : v;
         uv = vec2(u, v);
     }
-    const DImage img = s.images[t.image];
+    const DImage img = images[t.image];
     const int w = (int)img.width, h = (int)img.height;
     if (t.filter == SOL_GPU_FILTER_NEAREST) {
         // textures.cpp:23-28
         int x = clampi((int)(uv.x * (float)img.width), 0, w - 1);
         int y = clampi((int)(uv.y * (float)img.height), 0, h - 1);
-        return texel(s, img, x, y);
+        return texel(texels, img, x, y);
     }
     // Bilinear, textures.cpp:30-45
     float i = uv.x * (float)(img.width - 1);
@@ -77,10 +80,10 @@ __device__ SOL_TEX_FN Rgb image_color(const SceneView& s, const DTexture& t, Vec
     int y0 = clampi((int)j, 0, h - 1);
     int x1 = clampi(x0 + 1, 0, w - 1);
     int y1 = clampi(y0 + 1, 0, h - 1);
-    Rgb p00 = texel(s, img, x0, y0);
-    Rgb p10 = texel(s, img, x1, y0);
-    Rgb p01 = texel(s, img, x0, y1);
-    Rgb p11 = texel(s, img, x1, y1);
+    Rgb p00 = texel(texels, img, x0, y0);
+    Rgb p10 = texel(texels, img, x1, y0);
+    Rgb p01 = texel(texels, img, x0, y1);
+    Rgb p11 = texel(texels, img, x1, y1);
     return lerp(lerp(p00, p10, fu), lerp(p01, p11, fu), fv);
 }
 
@@ -88,21 +91,23 @@ __device__ SOL_TEX_FN Rgb image_color(const SceneView& s, const DTexture& t, Vec
 /// BSDFs (checked on the host when it is uploaded), so those branches are
 /// compiled out of the kernels built for such scenes: a smaller instruction
 /// footprint and fewer spills.  kShadeCall: full shading with the image lookup
-/// in one out-of-line copy, for kernels with many state registers (the
-/// multi-view megakernel on six textured scenes 923 -> 893 us; the single-view
-/// kernel is slower that way, 537 -> 553 us on a textured frame).
+/// in one out-of-line copy, for the megakernels (textured frames 701x389x7 597 ->
+/// 552 us, 1920x1080x8 4.06 -> 3.65 ms; the multi-view kernel on six textured
+/// scenes 983 -> 950 us).  kShadeFull: the same inlined, for the wavefront's
+/// shading stage, whose registers hold it.
 enum : int { kShadeFull, kShadeBasic, kShadeCall };
 
-__device__ __noinline__ inline Rgb image_color_call(const SceneView& s, const DTexture& t, Vec2 uv) {
-    return image_color(s, t, uv);
+__device__ __noinline__ inline Rgb image_color_call(const DImage* __restrict__ images, const float* __restrict__ texels,
+                                                    const DTexture& t, Vec2 uv) {
+    return image_color(images, texels, t, uv);
 }
 
 /// ColorTexture::sample_color.
 template <int kShade = kShadeFull>
 __device__ __forceinline__ Rgb tex_color(const SceneView& s, int id, Vec2 uv) {
     const DTexture& t = s.textures[id];
-    if (kShade == kShadeFull && t.kind == SOL_GPU_TEX_IMAGE) return image_color(s, t, uv);
-    if (kShade == kShadeCall && t.kind == SOL_GPU_TEX_IMAGE) return image_color_call(s, t, uv);
+    if (kShade == kShadeFull && t.kind == SOL_GPU_TEX_IMAGE) return image_color(s.images, s.texels, t, uv);
+    if (kShade == kShadeCall && t.kind == SOL_GPU_TEX_IMAGE) return image_color_call(s.images, s.texels, t, uv);
     return rgb(t.v[0], t.v[1], t.v[2]);
 }
 
