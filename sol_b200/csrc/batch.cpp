@@ -259,6 +259,7 @@ int refresh_scenes(SolGpuBatch* b) {
     if (!changed) return SOL_GPU_OK;
     cudaError_t e = cudaMemcpy(b->d_scenes, b->h_scenes.data(), sizeof(SceneView) * b->h_scenes.size(),
                                cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);   // renders may be on streams that do not wait for it
     if (e != cudaSuccess) return cuda_fail(e, "scene table upload");
     for (size_t i = 0; i < b->h_scenes.size() && i < kWfMaxScenes; ++i) b->wf_table.v[i] = b->h_scenes[i];
     destroy_graph(b);
@@ -593,6 +594,7 @@ int sol_gpu_batch_create(SolGpuScene* const* scenes, uint32_t num_scenes, const 
     }
     if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&b->d_sort_bins), 2 * sizeof(uint32_t) * kWfSortBins);
     if (e == cudaSuccess) e = cudaMemset(b->d_sort_bins, 0, 2 * sizeof(uint32_t) * kWfSortBins);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);   // renders may be on streams that do not wait for these
     if (e == cudaSuccess) e = allow_sort_smem();
     if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&b->h_ctr), sizeof(WfCounters));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking);

@@ -52,6 +52,7 @@ int check_fault(SolGpuScene* s) {
     if (e != cudaSuccess) return cuda_fail(e, "fault read");
     if (f == 0) return SOL_GPU_OK;
     cudaMemset(s->fault, 0, sizeof(unsigned int));
+    cudaStreamSynchronize(cudaStreamLegacy);   // before the next render, on whatever stream, records its own
     std::string msg = "a kernel self-check failed:";
     if (f & kFaultTraversalSteps) msg += " traversal exceeded its step bound or stack;";
     if (f & kFaultNodeIndex) msg += " BVH node index out of range;";
@@ -551,6 +552,7 @@ int sol_gpu_params_set(SolGpuScene* scene, const float* values) {
     if (e == cudaSuccess && scene->texel_count > 0)
         e = cudaMemcpy(scene->texels, values + scene->constants_count, sizeof(float) * scene->texel_count,
                        cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);   // as after the uploads of a new scene
     return e == cudaSuccess ? SOL_GPU_OK : cuda_fail(e, "params set");
 }
 
