@@ -271,7 +271,8 @@ def run_ours(args):
     st = pt.stats()
     rays_per_step = st.rays
 
-    # Algorithmic bytes per launch from the counting variant of the same render.
+    # Algorithmic bytes per launch from the counting variant of the same render, which
+    # takes shadow rays in the host's order (the timed kernels take the first child first).
     gscene.set_instrumented(True)
     pt.render_device(film.data_ptr(), w, h, base, spp, stream.cuda_stream)
     torch.cuda.synchronize()
@@ -345,6 +346,7 @@ def run_ours(args):
                              "peak_source": "measured here: L2-resident 64 MiB read (sol_b200/csrc/probe.cu)",
                              "bytes": "lts__t_bytes.sum of the stored one-pass ncu capture"},
                          "algorithmic_bytes_per_launch": alg_bytes,
+                         "algorithmic_bytes_from": "counting kernels, shadow rays in the host's child order",
                          "note": "per render call (megakernel + in-order sum pass)" if st.sample_chunk > 0
                                  else "per render call (one megakernel launch)"},
             "e2e": {"value": e2e, "unit": METRIC, "h2d_bytes_per_step": h2d_bytes,

@@ -270,7 +270,8 @@ int sol_gpu_scene_set_instrumented(SolGpuScene* scene, int instrumented);
  * running sums), held by the scene handle, so renders through one handle must
  * be ordered, e.g. issued on one stream.  AUTO (the default) picks SPLIT for
  * every render of more than one sample (measured faster at every image size),
- * PER_PIXEL for single samples or when the scratch cannot be allocated. */
+ * PER_PIXEL when the scratch cannot be allocated.  With AUTO and PER_PIXEL a
+ * single sample goes into the film directly, without scratch. */
 #define SOL_GPU_SCHEDULE_AUTO      0
 #define SOL_GPU_SCHEDULE_PER_PIXEL 1
 #define SOL_GPU_SCHEDULE_SPLIT     2

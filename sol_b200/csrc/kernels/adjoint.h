@@ -16,12 +16,19 @@ constexpr int kAdjointBlock = 128;
 /// hardly any spills), which only many paths in flight make up for.  So the
 /// build follows the path vertices of the call, counting each path with its
 /// length limit, per resident lane of the 4-block build.  Measured, adjoint at
-/// 4 / 8 / 16 blocks (us): textured Cornell, limit 16: 65.5k paths 488 / 597 /
-/// 905, 131k 903 / 737 / 1031, 262k 2140 / 1412 / 1299, 1.6M 17045 / 13023 /
-/// 10661; textured sphere field, limit 8: 33k 195 / 299 / 553, 131k 211 / 305 /
-/// 538, 262k 303 / 390 / 595.  Fused at 4 / 10 / 16 blocks: Cornell 65.5k 496 /
-/// 706 / 934, 262k 1834 / 1393 / 1357, 1M 7329 / 5293 / 5159; spheres 65.5k 202 /
-/// 380 / 536, 1M 945 / 865 / 1005, 2.2M 2276 / 1823 / 1860.
+/// 4 / 8 / 16 blocks (us; in brackets the vertices per lane, 4 blocks are taken up
+/// to 20, 8 up to 42): textured Cornell, limit 16: 65.5k paths 390 / 518 / 812
+/// (14), 73.7k 406 / 562 / 871 (16), 131k 647 / 612 / 908 (28), 197k 977 / 851 / 964
+/// (42), 262k 1346 / 1076 / 1072 (55), 1.6M 10256 / 7844 / 6032; textured sphere
+/// field, limit 8: 33k 198 / 306 / 557 (3), 131k 213 / 310 / 545 (14), 262k 285 / 407 /
+/// 614 (28), 410k 393 / 513 / 760 (43), 819k 542 / 612 / 851 (86), 1.6M 907 / 891 /
+/// 1191 (173).  Fused at 4 / 10 blocks: Cornell 65.5k 388 / 593 (14), 86k 526 / 642
+/// (18), 131k 697 / 696 (28), 262k 1424 / 1101 (55), 1M 5598 / 4072; spheres 147k
+/// 250 / 400 (16), 229k 311 / 479 (24), 492k 478 / 642 (52), 1M 771 / 787 (111), 2.2M
+/// 1812 / 1529 (228).  The limit says little about how long paths are, so no line
+/// serves both: these are the Cornell box's, whose paths use their limit; the
+/// sphere field's shorter paths would stay with the smaller build about four times
+/// as long (262k paths take 411 us instead of 285; one build for all took 636).
 enum class AdjointBuild { kSmall, kMiddle, kFull };
 constexpr int kAdjointSmallBlocks = 4, kAdjointMiddleBlocks = 8, kAdjointFullBlocks = 16;
 constexpr int kFusedFullBlocks = 10;   // the fused kernel's build for middle and full calls

@@ -100,8 +100,9 @@ struct GradSink {
 /// Sums `v` over the active lanes of the warp that pass the same `key`: the sums
 /// are on the lowest such lane, for which it returns true.  Every round, each
 /// lane that still holds a partial sum adds the next such lane's above it, and
-/// every other one drops out (after Westphal's warp-aggregated reduction), so
-/// one match and at most five rounds serve all values at once.
+/// every other one drops out (after Westphal, "Voting and Shuffling to Optimize
+/// Atomic Operations", NVIDIA Developer Blog, 2015), so one match and at most five
+/// rounds serve all values at once.
 template <typename T, int N>
 __device__ __forceinline__ bool reduce_by_key(unsigned long long key, T (&v)[N]) {
     const unsigned active = __activemask();
@@ -514,8 +515,8 @@ __device__ SOL_ADJ_OUTLINE void sweep(const SceneView& s, const VertexRec* rec, 
 /// Gradients of the first `n_shared` parameters (the constant textures) are
 /// gathered per block in shared memory and added into `grad` at the end.
 /// Only the first `lanes` lanes of a warp take items: a small call spreads its
-/// paths over more warps, where fewer wait for each other's branches (3,840
-/// paths of the textured Cornell box: 326 -> 224 us with one lane).
+/// paths over more warps, where fewer wait for each other's branches (a training
+/// step of 3,840 paths of the textured Cornell box: 499 -> 366 us with one lane).
 template <int kMinBlocks>
 __global__ void __launch_bounds__(kAdjointBlock, kMinBlocks)
 prb_adjoint(SceneView s, DCamera cam, DConfig cfg, uint64_t sample_index, uint32_t sample_count, uint32_t chunk,

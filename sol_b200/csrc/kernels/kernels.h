@@ -45,10 +45,14 @@ constexpr int kMegakernelViewsMinBlocks = SOL_MEGAKERNEL_VIEWS_MIN_BLOCKS;
 /// beyond 16 are cut short by the roulette).  Fewer paths than that are under
 /// way together from the start, and the launch lasts as long as its longest
 /// paths do, which the 6-block build, spilling hardly at all, traces sooner.
-/// Measured, 6 against 12 blocks (us): Cornell, limit 16: 25.6k paths x 4 278 /
-/// 348, 205k 394 / 403, 262k 496 / 483, 480k 755 / 700, 1M 1530 / 1353; sphere
-/// fields, limit 8: 230k 392 / 432, 410k 252 / 281, 518k 217 / 229, textured
-/// 240k 233 / 253; 1M triangles, 2M paths 1037 / 993, 8M 3281 / 2848.
+/// Measured, 6 against 12 blocks (us; in brackets the vertices per lane, 12 blocks
+/// are taken above 16): Cornell, limit 16: 102k paths 237 / 309 (7), 205k 344 /
+/// 362 (14), 262k 412 / 416 (18), 480k 650 / 614 (34), 1M 1281 / 1144 (74); sphere
+/// fields, limit 8: 230k 294 / 321 (8), 410k 270 / 291 (14), 518k 221 / 238 (18),
+/// 922k 248 / 296 (32), textured 518k 312 / 348 (18); 1M triangles, 2M paths
+/// 1150 / 1101 (73), 8M 3576 / 3123.  The length limit says little about how long
+/// paths are, so no line serves both: this one is the Cornell box's, whose paths
+/// use their limit, and costs short ones up to 19 % between 0.45M and 2M of them.
 constexpr uint64_t kMegakernelFullVerticesPerLane = 16;
 constexpr uint32_t kMegakernelMinCountedLen = 8, kMegakernelMaxCountedLen = 16;
 constexpr int kTraceBlock = 64;

@@ -281,10 +281,10 @@ __device__ __forceinline__ void set_cost(Treelet& w, int s, float best, int bp, 
 /// 6 leaves four lanes per subset, all 7 on the whole warp.  One thread per
 /// treelet took about 1,000 partitions one after another, with its tables in
 /// local memory, along the whole chain of nodes from the triangles to the root:
-/// three passes over 65,546 triangles 9.7 ms (the
-/// whole build 13.6 ms, now 5.5; 262,154 triangles 32.5 -> 15.3, 1,048,586 70 ->
-/// 22.7).  Partitions are compared in the
-/// same order of preference, so the tree is the same.
+/// three passes over 65,546 triangles 9.7 ms (the whole build 13.6 -> 5.5 ms;
+/// 262,154 triangles 32.5 -> 15.3, 1,048,586 70 -> 22.7, before build_lbvh took its
+/// arrays in one allocation).  Partitions are compared in the same order of
+/// preference, so the tree is the same.
 __device__ void restructure(const Tree& t, int root, float root_cost, Treelet& w) {
     const unsigned all = 0xffffffffu;
     const int lane = (int)(threadIdx.x & 31u);
@@ -641,8 +641,9 @@ cudaError_t build_lbvh(const float* vertices, const uint32_t* indices, const flo
     unsigned int *arrived = nullptr, *depth = nullptr, *fail = nullptr;
     // All working arrays in one allocation: allocating and freeing them one by
     // one took longer than the kernels (with the mesh arrays and the scene's
-    // small tables in one allocation each, creation 18.1 -> 6.6 ms at 262,154
-    // triangles, 46.2 -> 12.7 ms at 1,048,586).
+    // small tables in one allocation each, creation 18.1 -> 6.3 ms at 262,154
+    // triangles, 46.2 -> 12.2 ms at 1,048,586, of which the build with its
+    // uploads is 5.4 and 11.1).
     size_t temp_bytes = 0;
     cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys, keys_sorted, order, order_sorted, n, 0, 63, stream);
     void *work = nullptr, *temp = nullptr;

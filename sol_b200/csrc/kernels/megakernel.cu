@@ -10,8 +10,9 @@
 // per-pixel sum in SoL's sample order and the result bit-identical to the host.
 //
 // Single samples take the lean kernel below.  Renders of more than one sample
-// use the split schedule (the host's AUTO choice), also on the lean kernel: a work item is one (pixel, sample), so the samples of a pixel
-// run on different lanes; each writes its path's colour (0 + colour, as the
+// use the split schedule (the host's AUTO choice), also on the lean kernel: a
+// work item is one (pixel, sample), so the samples of a pixel run on different
+// lanes; each writes its path's colour (0 + colour, as the
 // per-pixel sum starts) to a scratch plane of its sample, and sum_samples adds
 // each pixel's colours in sample order, which is the same sequence of
 // additions as the per-pixel loop and gives the same bits.
@@ -196,8 +197,8 @@ pt_megakernel_lean(SceneView s, DCamera cam, DConfig cfg, uint64_t sample_index,
     uint32_t n_paths = 0, n_rays = 0, n_shadow = 0;
     LocalStack stack;
     // One bounce per iteration; the warp's idle lanes claim new items together
-    // once at least `regen` of them are idle (or no lane has a path), so lanes neither wait for the warp's longest path nor drift apart
-    // one by one.  Every lane stays in the loop until the whole warp is done
+    // once at least `regen` of them are idle (or no lane has a path), so lanes
+    // neither wait for the warp's longest path nor drift apart one by one.  Every lane stays in the loop until the whole warp is done
     // (the exit test is a warp-uniform vote), so the full-warp votes and the
     // barrier see all 32 lanes; every iteration either advances a live path by
     // one bounce or claims items, so the loop ends with the items.
@@ -475,8 +476,7 @@ auto lean_fn(bool full, bool basic) {
 /// give every path a lane with fewer (a power of two).  Paths that share a
 /// warp wait for each other's divergent branches, so a render of a few
 /// thousand paths is done sooner spread over all resident warps: 64x48 Cornell
-/// preview 210 -> 128 us (one lane), 128x128 184 -> 165 (8), 200x120 textured
-/// 157 -> 126 (8).
+/// preview 196 -> 127 us (one lane), 128x128x2 230 -> 215 (16).
 uint32_t lanes_per_warp(uint64_t paths, int grid) {
     const uint64_t warps = (uint64_t)grid * (kMegakernelBlock / 32);
     uint32_t lanes = 1;

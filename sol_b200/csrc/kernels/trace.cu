@@ -14,12 +14,12 @@ namespace {
 /// One ray per thread, on the first `lanes` lanes of each warp (a power of two):
 /// a batch that the resident warps could hold with fewer lanes is spread over
 /// them, since the rays of a warp mostly trace one after another (1,000 closest
-/// hits 19.3 -> 14.3 us; from 8 lanes on the longest ray alone decides, 20,000
-/// take 36.9 us with 32 and 37.4 with 8).  64-thread blocks leave the SM as soon
-/// as their own longest ray ends; the occupancies (16 blocks: 64 registers, 24:
-/// 40) are the fastest measured: closest hits of 300k rays 38.8 us against 43.0 at
-/// 24 and 47.1 at 32 blocks, shadow rays 124.3 us against 125.6 at 16 and 131.6
-/// at 32; 128-thread blocks 38.9 and 125.6.
+/// hits 25.2 -> 20.1 us with the launch; from 8 lanes on the longest ray alone
+/// decides, 20,000 take 43 us with 32 as with 8).  64-thread blocks leave the SM as
+/// soon as their own longest ray ends.  Occupancies (16 blocks: 64 registers, 24:
+/// 40): closest hits of 300k rays 44.7 us against 46.9 at 24 and 49.6 at 32 blocks
+/// (4M rays 381, 359, 366), 1.5M shadow rays 123 us against 124 at 16 and 139 at 32;
+/// 128-thread blocks 47.0 and 123.
 template <bool kAnyHit>
 __global__ void __launch_bounds__(kTraceBlock, kAnyHit ? 24 : 16)
 trace_rays(SceneView s, const SolGpuRay* __restrict__ rays, uint32_t count, SolGpuHit* __restrict__ hits, uint32_t lanes) {

@@ -253,8 +253,8 @@ __device__ __forceinline__ WfStack make_stack() { return WfStack{}; }
 /// with fewer, only that many lanes of each warp (a power of two) take rays: the
 /// last bounces of a batch leave a few thousand incoherent rays, which a warp
 /// of 32 traces nearly one after another (24 views, bounces 10 to 16: 120-200
-/// us per traversal stage; the batch 8.77 -> 8.38 ms, four small views 0.97 ->
-/// 0.69 ms, twenty single-sample views 1.06 -> 0.93 ms).
+/// us per traversal stage; the batch 8.28 -> 7.99 ms, four small views 0.80 ->
+/// 0.59 ms, twenty single-sample views 0.99 -> 0.87 ms).
 template <bool kAnyHit, class Fetch, class Finish>
 __device__ __forceinline__ void trace_queue(const WfSceneTable& scenes, uint32_t n, uint32_t* fetch_counter,
                                             int refill_below, Fetch fetch, Finish finish,

@@ -27,11 +27,11 @@ constexpr int kWfRefillBelow = SOL_WF_REFILL_BELOW;
 /// 3 (up to 80 registers, nothing spilled): the stages are chains of dependent
 /// node fetches that spilling (6 blocks, 40 registers) lengthens, and every
 /// bounce launches the full grid, so fewer blocks also cost less where the
-/// queues are short.  24 views (19M paths) of 262k triangles 8.89 ms at 6
-/// blocks, 8.65 at 5, 8.56 at 4, 8.52 at 3.  Scenes that L2 does not hold beside
-/// the queues (kWfCachedSceneBytes of nodes and triangles) wait for memory
-/// instead, which more warps hide: the same views of 1M triangles 12.43, 12.24,
-/// 12.58 and 12.98 ms, of 4.2M 25.28, 25.32, 26.64 and 28.71 ms.
+/// queues are short.  Scenes that L2 does not hold beside the queues
+/// (kWfCachedSceneBytes of nodes and triangles) wait for memory instead, which
+/// more warps hide.  24 views (19M paths) at 3 / 5 blocks: 28 MB 8.31 / 8.44 ms, 42
+/// MB 8.85 / 8.81, 56 MB 9.92 / 9.64, 84 MB 11.19 / 10.70, 112 MB 12.66 / 12.00, 448
+/// MB 27.9 / 24.8.
 constexpr int kWfTraceMinBlocks = SOL_WF_TRACE_MIN_BLOCKS;
 constexpr int kWfTraceLargeMinBlocks = 5;
 constexpr uint64_t kWfCachedSceneBytes = 48ull << 20;
